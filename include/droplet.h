@@ -297,9 +297,11 @@ const char *dl_flow_last_error(const dl_flow *f);
 int dl_flow_set_stream(dl_flow *f, void *stream);
 int dl_flow_sync(dl_flow *f);
 /* Device time of the flow steps taken since the last call, averaged per step (ms), in
- * four parts: the inverse cuFFT transform, the cross-product kernel (with the droplet
- * field copy), the forward cuFFT transform, and the update kernels (update, forcing,
- * finish); CUDA events when enabled (the reference times the flow step as a whole,
+ * four parts: the inverse transform, the cross-product kernel (with the droplet
+ * field copy), the forward transform, and the update kernels (update, forcing,
+ * finish).  On the grids with passes of their own (2^a and 3 * 2^a, 32 to 512) the x
+ * transforms of both directions belong to the second part and the inverse z transforms of
+ * the next step to the fourth.  CUDA events when enabled (the reference times the flow step as a whole,
  * turb.f90:734-755).  Returns the averages, then enables (1) or disables (0) the timing
  * and resets it.  Synchronises. */
 int dl_flow_timing(dl_flow *f, int enable, double *ms4, int *steps);

@@ -2,26 +2,30 @@
 // flowlib.f90:180-562 and the transforms of mpifft.f90:81-198), FP64 as the reference.
 //
 // The reference's distributed 3D transforms (FFTW 1D passes + MPI transposes, forward
-// normalised by 1/n per pass) become single-GPU cuFFT 3D transforms (Z2D / D2Z, batched
-// over components); the forward 1/n^3 is applied inside the update kernel.  Spectral
-// arrays use cuFFT's R2C layout, component c at c * M, mode (kz, ky, kx >= 0) at
-// (z * n + y) * (n/2 + 1) + x, complex (re, im) interleaved; physical arrays are n^3,
-// x fastest.
+// normalised by 1/n per pass) run on one GPU; the forward 1/n^3 is applied in the update.
+// Spectral arrays of the interface have component c at c * n * n * (n/2 + 1), mode
+// (kz, ky, kx >= 0) at (z * n + y) * (n/2 + 1) + x, complex (re, im) interleaved; physical arrays
+// are n^3, x fastest.
 //
-// One step:
-//   C2R of [curl u^, u^] (batched, 6 transforms) -> physical omega, u  (turb.f90:506-539;
-//     u is the field the particle substep of this step interpolates)
-//   k_cross: N = u x omega in place of omega                           (turb.f90:634-637)
-//   D2Z of N (3 transforms)                                            (turb.f90:644-646)
-//   k_update: dealias N, Crank-Nicolson viscous + AB2 nonlinear update, stochastic
-//     forcing (supforSTH), projection, division by (1 + nu dt/2 k^2), N_old = N
-//                                                                      (turb.f90:648-676)
-//   k_force_det (forcing = 1): shells 1 and 2 rescaled to force(1:2)   (flowlib.f90:195-229)
-//   k_finish: symmetrize (zero mean, Nyquist planes, Hermitian kx = 0 plane), dealias,
-//     and the transform inputs [curl u^, u^] of the next step          (flowlib.f90:180-334)
+// One step, whichever way it is transformed:
+//   [curl u^, u^] -> physical omega, u (6 transforms; u is the field the particle substep of
+//     this step interpolates)                                        (turb.f90:506-539)
+//   N = u x omega                                                    (turb.f90:634-637)
+//   N -> N^ (3 transforms)                                           (turb.f90:644-646)
+//   dealias N^, Crank-Nicolson viscous + AB2 nonlinear update, stochastic forcing
+//     (supforSTH), projection, division by (1 + nu dt/2 k^2), N_old = N^ (turb.f90:648-676)
+//   forcing = 1: shells 1 and 2 rescaled to force(1:2)               (flowlib.f90:195-229)
+//   symmetrize (zero mean, Nyquist planes, Hermitian kx = 0 plane), dealias, and the transform
+//     inputs [curl u^, u^] of the next step                          (flowlib.f90:180-334)
+// Grids 2^a and 3 * 2^a from 32 to 512 take the passes of dl_flow_passes.cuh, which transform
+// along one direction each, only inside the dealiasing sphere, with the cross product between
+// the two x transforms in shared memory: 256^3 2.12 -> 1.37 ms, 512^3 18.5 -> 11.4 ms,
+// 64^3 86 -> 48 us, 192^3 1.02 -> 0.59 ms.  Other grids take cuFFT's 3D transforms (Z2D / D2Z, batched
+// over components) with kernels for the cross product, the update and the finish.
 // Decision on a reference quirk: with one rank, symmetrize's test idlocalZ .eq. nprocZ/2
 // (flowlib.f90:253) is true for the rank holding ky = 0 and would zero the ky = 0 plane;
 // every multi-rank run zeroes the ky = n/2 plane there, which is what this code does.
+#include "dl_fft.cuh"
 #include "dl_internal.cuh"
 
 #include <cufft.h>
@@ -30,13 +34,16 @@
 #include <cmath>
 #include <cstring>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 namespace {
 
 struct Grid {
     int n, nh;          // n, n/2 + 1
-    int64_t M;          // complex modes per component
+    int px;             // row pitch of the spectral state (modes; kx >= nh unused)
+    int yz;             // its rows in order [y][z] rather than [z][y]
+    int64_t M;          // complex modes per component, n * n * px
     int nek;            // dealiasing shell: int(n/2 - 1.5) (turb.f90:303-304)
 };
 
@@ -44,16 +51,21 @@ __device__ __forceinline__ void mode_of(const Grid &G, int64_t m, int &x, int &y
                                         double &kz)
 {
     if (G.M <= 0x7fffffff) {   // 32-bit index arithmetic (every grid up to 1024^3)
-        const unsigned mu = (unsigned)m, nh = (unsigned)G.nh, nn = (unsigned)G.n;
-        const unsigned zy = mu / nh;
-        x = (int)(mu - zy * nh);
+        const unsigned mu = (unsigned)m, px = (unsigned)G.px, nn = (unsigned)G.n;
+        const unsigned zy = mu / px;
+        x = (int)(mu - zy * px);
         z = (int)(zy / nn);
         y = (int)(zy - (unsigned)z * nn);
     } else {
-        x = (int)(m % G.nh);
-        const int64_t zy = m / G.nh;
+        x = (int)(m % G.px);
+        const int64_t zy = m / G.px;
         y = (int)(zy % G.n);
         z = (int)(zy / G.n);
+    }
+    if (G.yz) {
+        const int s = y;
+        y = z;
+        z = s;
     }
     kx = (double)x;
     ky = (double)(y < G.n / 2 + 1 ? y : y - G.n);
@@ -144,10 +156,9 @@ struct UpdArgs {
 __device__ __forceinline__ void emit_mode(const Grid &G, int64_t m, double kx, double ky, double kz,
                                           const double2 *v, double2 *u, double2 *work)
 {
-    for (int c = 0; c < 3; c++) {
-        u[c * G.M + m] = v[c];
-        work[(3 + c) * G.M + m] = v[c];
-    }
+    for (int c = 0; c < 3; c++) u[c * G.M + m] = v[c];
+    if (!work) return;
+    for (int c = 0; c < 3; c++) work[(3 + c) * G.M + m] = v[c];
     // curl: w = k x u, multiplied by i: (re, im) -> (-im, re)
     const double2 w[3] = {make_double2(ky * v[2].x - kz * v[1].x, ky * v[2].y - kz * v[1].y),
                           make_double2(kz * v[0].x - kx * v[2].x, kz * v[0].y - kx * v[2].y),
@@ -270,6 +281,7 @@ __device__ __forceinline__ void finish_mode(const Grid &G, int64_t m, double2 *u
     int x, y, z;
     double kx, ky, kz;
     mode_of(G, m, x, y, z, kx, ky, kz);
+    if (x >= G.nh) return;
     const int h = G.n / 2;
     const bool zero = (x == 0 && y == 0 && z == 0) || x == h || y == h || z == h ||
                       ik2_of(kx * kx + ky * ky + kz * kz) > G.nek;
@@ -286,7 +298,7 @@ __device__ __forceinline__ void finish_mode(const Grid &G, int64_t m, double2 *u
     }
     // kx = 0: the thread of the lower index of each conjugate pair averages both
     const int yp = (G.n - y) % G.n, zp = (G.n - z) % G.n;
-    const int64_t mp = ((int64_t)zp * G.n + yp) * G.nh;
+    const int64_t mp = (G.yz ? (int64_t)yp * G.n + zp : (int64_t)zp * G.n + yp) * G.px;
     if (mp < m) return;
     double2 vp[3];
     for (int c = 0; c < 3; c++) {
@@ -310,7 +322,7 @@ __global__ void k_finish_low(Grid G, double2 *u, double2 *work)
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= 3 * (int64_t)G.n * G.n) return;
     const int64_t zy = t / 3;
-    finish_mode(G, zy * G.nh + (t - 3 * zy), u, work);
+    finish_mode(G, zy * G.px + (t - 3 * zy), u, work);
 }
 
 // energy per shell ik2 (kx = 0 modes count half): partial sums per CTA, in order
@@ -324,7 +336,7 @@ __global__ void k_spectrum(Grid G, const double2 *u, int nshell, double *part)
         double kx, ky, kz;
         mode_of(G, m, x, y, z, kx, ky, kz);
         const int s = ik2_of(kx * kx + ky * ky + kz * kz);
-        if (s >= nshell) continue;
+        if (s >= nshell || x >= G.nh) continue;
         double t = 0.0;
         for (int c = 0; c < 3; c++) {
             const double2 v = u[c * G.M + m];
@@ -348,7 +360,8 @@ __global__ void k_pack(int n, const double *v, int64_t py, int64_t pz, double *o
     out[i] = v[x + py * y + pz * z];
 }
 
-// plain u^ <- u^_raw / n^3 then projection (turb.f90 initial state / restart path)
+// plain u^ <- u^_raw / n^3 then projection (turb.f90 initial state / restart path); raw in
+// cuFFT's layout (rows of nh modes)
 __global__ void k_project_scaled(Grid G, const double2 *raw, double inv_n3, double2 *u)
 {
     const int64_t m = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -356,10 +369,12 @@ __global__ void k_project_scaled(Grid G, const double2 *raw, double inv_n3, doub
     int x, y, z;
     double kx, ky, kz;
     mode_of(G, m, x, y, z, kx, ky, kz);
+    if (x >= G.nh) return;
     const double k2 = k2_of(kx, ky, kz);
+    const int64_t rows = (int64_t)G.n * G.n, row = (int64_t)z * G.n + y;
     double2 v[3];
     for (int c = 0; c < 3; c++) {
-        v[c] = raw[c * G.M + m];
+        v[c] = raw[(c * rows + row) * G.nh + x];
         v[c].x *= inv_n3;
         v[c].y *= inv_n3;
     }
@@ -369,6 +384,20 @@ __global__ void k_project_scaled(Grid G, const double2 *raw, double inv_n3, doub
     for (int c = 0; c < 3; c++) u[c * G.M + m] = make_double2(v[c].x - kk[c] * tr, v[c].y - kk[c] * ti);
 }
 
+// N_old <- 0 outside the sphere: what a step leaves there (a state set from outside may not)
+__global__ void k_dealias(Grid G, double2 *v)
+{
+    const int64_t m = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (m >= G.M) return;
+    int x, y, z;
+    double kx, ky, kz;
+    mode_of(G, m, x, y, z, kx, ky, kz);
+    if (ik2_of(kx * kx + ky * ky + kz * kz) > G.nek)
+        for (int c = 0; c < 3; c++) v[c * G.M + m] = make_double2(0.0, 0.0);
+}
+
+#include "dl_flow_passes.cuh"
+
 }  // namespace
 
 struct dl_flow {
@@ -377,7 +406,14 @@ struct dl_flow {
     Grid G;
     cudaStream_t stream = nullptr, own_stream = nullptr;
     double2 *u = nullptr, *nold = nullptr, *work = nullptr;
-    double *phys = nullptr;      // [6][n^3]: omega (then N), u
+    double *phys = nullptr;      // cuFFT path: [6][n^3]: omega (then N), u
+    double *vel = nullptr;       // [3][n^3]: u (cuFFT path: within phys)
+    // grids with passes of their own (dl_flow_passes.cuh); work is then W
+    int fast = 0;
+    double2 *planes = nullptr;   // P
+    double2 *box = nullptr;      // modes of the deterministic forcing
+    double2 *tw = nullptr, *tw_wide = nullptr;   // twiddles of the Narrow plan (x) and the Wide one (y, z)
+    int nold_dirty = 0;          // N_old may hold modes outside the sphere
     double *afor = nullptr;      // device copy of the stochastic forcing amplitudes
     double *spec_part = nullptr;
     cufftHandle c2r = 0, r2c = 0;
@@ -527,11 +563,166 @@ __global__ void k_dissip_acc(int64_t n3, const double *__restrict__ t, int which
     e[i] = a;
 }
 
-int finish(dl_flow *f)
+// ---- the passes of dl_flow_passes.cuh, per grid size ---------------------------------------
+template <int N>
+struct Passes {
+    static constexpr int H = N / 2, YS = 8 * slot_len<dlfft::Wide<N>>() * 16, YT = 8 * dlfft::Wide<N>::T;
+
+    static cudaError_t setup()
+    {
+        const struct { const void *k; int bytes; } a[] = {
+            {(const void *)k_ypass<N, 1>, YS}, {(const void *)k_ypass<N, -1>, YS},
+            {(const void *)k_xpass<N, X_STEP>, x_smem<N>()}, {(const void *)k_xpass<N, X_EMIT32>, x_smem<N>()},
+            {(const void *)k_xpass<N, X_EMIT64>, x_smem<N>()}, {(const void *)k_xpass<N, X_DISS>, x_smem<N>()},
+            {(const void *)k_zforward<N>, YS}, {(const void *)k_zinverse<N, Z_STATE>, YS},
+            {(const void *)k_zinverse<N, Z_STRAIN>, YS}};
+        for (const auto &q : a) {
+            const cudaError_t e = cudaFuncSetAttribute(q.k, cudaFuncAttributeMaxDynamicSharedMemorySize, q.bytes);
+            if (e != cudaSuccess) return e;
+        }
+        return cudaSuccess;
+    }
+    // twiddles w^(m q) of the stages after the first, as dlfft::butterflies reads them
+    template <class P>
+    static std::vector<double2> table()
+    {
+        std::vector<double2> t;
+        const int R[3] = {P::R0, P::R1, P::R2};
+        int ns = R[0];
+        for (int s = 1; s < P::S; s++) {
+            for (int m = 1; m < R[s]; m++)
+                for (int q = 0; q < ns; q++) {
+                    const long double a =
+                        2.0L * 3.14159265358979323846264338327950288L * ((int64_t)m * q % (ns * R[s])) / (ns * R[s]);
+                    t.push_back(make_double2((double)cosl(a), (double)sinl(a)));
+                }
+            ns *= R[s];
+        }
+        return t;
+    }
+    static std::vector<double2> wide() { return table<dlfft::Wide<N>>(); }
+    static std::vector<double2> narrow() { return table<XPlan<N>>(); }
+    static void ypass(dl_flow *f, bool inverse)
+    {
+        if (inverse) k_ypass<N, 1><<<dim3(H / 8, N, 6), YT, YS, f->stream>>>(f->work, f->planes, f->G.nek, f->tw_wide);
+        else k_ypass<N, -1><<<dim3(H / 8, N, 3), YT, YS, f->stream>>>(f->work, f->planes, f->G.nek, f->tw_wide);
+    }
+    static void xpass(dl_flow *f, int mode, const XArgs &A)
+    {
+        const dim3 grid(N / (2 * x_units<N>()), N);
+        constexpr int T = x_threads<N>(), S = x_smem<N>();
+        if (mode == X_STEP) k_xpass<N, X_STEP><<<grid, T, S, f->stream>>>(A);
+        else if (mode == X_EMIT32) k_xpass<N, X_EMIT32><<<grid, T, S, f->stream>>>(A);
+        else if (mode == X_EMIT64) k_xpass<N, X_EMIT64><<<grid, T, S, f->stream>>>(A);
+        else k_xpass<N, X_DISS><<<grid, T, S, f->stream>>>(A);
+    }
+    static void zforward(dl_flow *f, const ZArgs &A) { k_zforward<N><<<dim3(H / 8, N, 3), YT, YS, f->stream>>>(A); }
+    static void zinverse(dl_flow *f, const ZArgs &A, bool strain)
+    {
+        const dim3 grid(H / 8, 6, N);
+        if (strain) k_zinverse<N, Z_STRAIN><<<grid, YT, YS, f->stream>>>(A);
+        else k_zinverse<N, Z_STATE><<<grid, YT, YS, f->stream>>>(A);
+    }
+};
+
+// calls f with the Passes of grid size n
+template <typename F>
+void with_passes(int n, F f)
 {
-    k_finish<<<blocks(f->G.M, 256), 256, 0, f->stream>>>(f->G, f->u, f->work);
+    switch (n) {
+    case 32: f(Passes<32>()); break;
+    case 48: f(Passes<48>()); break;
+    case 64: f(Passes<64>()); break;
+    case 96: f(Passes<96>()); break;
+    case 128: f(Passes<128>()); break;
+    case 192: f(Passes<192>()); break;
+    case 256: f(Passes<256>()); break;
+    case 384: f(Passes<384>()); break;
+    case 512: f(Passes<512>()); break;
+    default: break;
+    }
+}
+
+ZArgs z_args(dl_flow *f)
+{
+    ZArgs A;
+    std::memset(&A, 0, sizeof(A));
+    A.W = f->work;
+    A.u = f->u;
+    A.nold = f->nold;
+    A.box = f->box;
+    A.n = f->G.n;
+    A.px = f->G.px;
+    A.nek = f->G.nek;
+    A.nu = f->p.nu;
+    A.dt = f->p.dt;
+    A.inv_n3 = 1.0 / ((double)f->G.n * f->G.n * f->G.n);
+    A.tw = f->tw_wide;
+    return A;
+}
+
+XArgs x_args(dl_flow *f)
+{
+    XArgs A;
+    std::memset(&A, 0, sizeof(A));
+    A.P = f->planes;
+    A.nek = f->G.nek;
+    A.vel = f->vel;
+    A.tw = f->tw;
+    return A;
+}
+
+// W from the state
+int transform_state(dl_flow *f, bool strain)
+{
+    const ZArgs A = z_args(f);
+    with_passes(f->G.n, [&](auto P) { P.zinverse(f, A, strain); });
     f->launches++;
     FCUDA(f, cudaGetLastError());
+    return 0;
+}
+
+int finish(dl_flow *f)
+{
+    k_finish<<<blocks(f->G.M, 256), 256, 0, f->stream>>>(f->G, f->u, f->fast ? nullptr : f->work);
+    f->launches++;
+    FCUDA(f, cudaGetLastError());
+    return f->fast ? transform_state(f, false) : 0;
+}
+
+// spectral state between the caller's layout (rows [z][y] of nh modes) and the context's
+__global__ void k_layout(Grid G, double2 *state, double2 *packed, int in)
+{
+    const int64_t m = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (m >= G.M) return;
+    int x, y, z;
+    double kx, ky, kz;
+    mode_of(G, m, x, y, z, kx, ky, kz);
+    if (x >= G.nh) return;
+    const int64_t q = ((int64_t)z * G.n + y) * G.nh + x;
+    if (in) state[m] = packed[q];
+    else packed[q] = state[m];
+}
+
+// all three components, caller <-> state, one at a time through a buffer where the layouts differ
+int copy_state(dl_flow *f, double2 *state, void *caller, bool in, cudaMemcpyKind k)
+{
+    const int64_t packed = (int64_t)f->G.n * f->G.n * f->G.nh;
+    if (!f->fast) {
+        const size_t b = sizeof(double2) * 3 * packed;
+        FCUDA(f, in ? cudaMemcpyAsync(state, caller, b, k, f->stream) : cudaMemcpyAsync(caller, state, b, k, f->stream));
+        return 0;
+    }
+    double2 *tmp = nullptr;
+    FCUDA(f, cudaMallocAsync((void **)&tmp, sizeof(double2) * packed, f->stream));
+    for (int c = 0; c < 3; c++) {
+        double2 *mine = static_cast<double2 *>(caller) + c * packed;
+        if (in) FCUDA(f, cudaMemcpyAsync(tmp, mine, sizeof(double2) * packed, k, f->stream));
+        k_layout<<<blocks(f->G.M, 256), 256, 0, f->stream>>>(f->G, state + c * f->G.M, tmp, in);
+        FCUDA(f, cudaGetLastError());
+        if (!in) FCUDA(f, cudaMemcpyAsync(mine, tmp, sizeof(double2) * packed, k, f->stream));
+    }
+    FCUDA(f, cudaFreeAsync(tmp, f->stream));
     return 0;
 }
 
@@ -550,7 +741,10 @@ extern "C" int dl_flow_create(const dl_flow_params *p, dl_flow **out)
     const int n = p->n;
     f->G.n = n;
     f->G.nh = n / 2 + 1;
-    f->G.M = (int64_t)n * n * f->G.nh;
+    f->fast = dlfft::supported(n);
+    f->G.yz = f->fast;
+    f->G.px = f->fast ? n / 2 + 8 : f->G.nh;   // fast: rows of whole 128-byte lines
+    f->G.M = (int64_t)n * n * f->G.px;
     f->G.nek = (int)(n / 2 - 1.5);
     std::memset(f->b, 0, sizeof(f->b));
     std::memset(f->ivf, 0, sizeof(f->ivf));
@@ -567,23 +761,49 @@ extern "C" int dl_flow_create(const dl_flow_params *p, dl_flow **out)
         cudaEventCreateWithFlags(&f->ev_used, cudaEventDisableTiming) != cudaSuccess)
         return fail(DL_E_CUDA);
     const int64_t n3 = (int64_t)n * n * n;
+    const int64_t wplane = (int64_t)n * (n / 2) + WPAD;
     if (cudaMalloc(&f->u, sizeof(double2) * 3 * f->G.M) != cudaSuccess ||
         cudaMalloc(&f->nold, sizeof(double2) * 3 * f->G.M) != cudaSuccess ||
-        cudaMalloc(&f->work, sizeof(double2) * 6 * f->G.M) != cudaSuccess ||
-        cudaMalloc(&f->phys, sizeof(double) * 6 * n3) != cudaSuccess ||
+        cudaMalloc(&f->work, sizeof(double2) * 6 * (f->fast ? wplane * n : f->G.M)) != cudaSuccess ||
+        cudaMalloc(&f->phys, sizeof(double) * (f->fast ? 3 : 6) * n3) != cudaSuccess ||
         cudaMalloc(&f->afor, sizeof(double) * 450) != cudaSuccess ||
         cudaMalloc(&f->spec_part, sizeof(double) * 296 * 1024) != cudaSuccess)
         return fail(DL_E_ALLOC);
     cudaMemsetAsync(f->u, 0, sizeof(double2) * 3 * f->G.M, f->stream);
     cudaMemsetAsync(f->nold, 0, sizeof(double2) * 3 * f->G.M, f->stream);
+    f->vel = f->fast ? f->phys : f->phys + 3 * n3;
+    if (f->fast) {
+        std::vector<double2> tab;
+        size_t nt = 0;
+        cudaError_t e = cudaSuccess;
+        with_passes(n, [&](auto P) {
+            e = P.setup();
+            tab = P.narrow();
+            nt = tab.size();
+            const std::vector<double2> w = P.wide();
+            tab.insert(tab.end(), w.begin(), w.end());
+        });
+        if (e != cudaSuccess) return fail(DL_E_CUDA);
+        if (cudaMalloc(&f->planes, sizeof(double2) * 3 * n3) != cudaSuccess ||   // [6][n][n][n/2]
+            cudaMalloc(&f->box, sizeof(double2) * 3 * 75) != cudaSuccess ||
+            cudaMalloc(&f->tw, sizeof(double2) * tab.size()) != cudaSuccess)
+            return fail(DL_E_ALLOC);
+        if (cudaMemcpyAsync(f->tw, tab.data(), sizeof(double2) * tab.size(), cudaMemcpyHostToDevice, f->stream) !=
+                cudaSuccess ||
+            cudaStreamSynchronize(f->stream) != cudaSuccess)
+            return fail(DL_E_CUDA);
+        f->tw_wide = f->tw + nt;
+    }
     int dims[3] = {n, n, n};
-    if (cufftPlanMany(&f->c2r, 3, dims, nullptr, 1, 0, nullptr, 1, 0, CUFFT_Z2D, 6) != CUFFT_SUCCESS)
-        return fail(DL_E_ALLOC);
-    f->have_c2r = true;
+    if (!f->fast) {
+        if (cufftPlanMany(&f->c2r, 3, dims, nullptr, 1, 0, nullptr, 1, 0, CUFFT_Z2D, 6) != CUFFT_SUCCESS)
+            return fail(DL_E_ALLOC);
+        f->have_c2r = true;
+        cufftSetStream(f->c2r, f->stream);
+    }
     if (cufftPlanMany(&f->r2c, 3, dims, nullptr, 1, 0, nullptr, 1, 0, CUFFT_D2Z, 3) != CUFFT_SUCCESS)
         return fail(DL_E_ALLOC);
     f->have_r2c = true;
-    cufftSetStream(f->c2r, f->stream);
     cufftSetStream(f->r2c, f->stream);
     *out = f;
     return 0;
@@ -596,7 +816,8 @@ extern "C" int dl_flow_destroy(dl_flow *f)
     if (f->have_c2r) cufftDestroy(f->c2r);
     if (f->have_r2c) cufftDestroy(f->r2c);
     if (f->have_c2r1) cufftDestroy(f->c2r1);
-    void *ptrs[] = {f->u, f->nold, f->work, f->phys, f->afor, f->spec_part, f->diss_spec, f->diss_phys, f->diss};
+    void *ptrs[] = {f->u, f->nold, f->work, f->phys, f->afor, f->spec_part, f->diss_spec, f->diss_phys, f->diss,
+                    f->planes, f->box, f->tw};
     for (void *q : ptrs)
         if (q) cudaFree(q);
     for (int i = 0; i < 5 * dl_flow::NTS; i++)
@@ -617,7 +838,7 @@ extern "C" int dl_flow_set_stream(dl_flow *f, void *stream)
 {
     if (!f) return DL_E_ARG;
     f->stream = stream ? (cudaStream_t)stream : f->own_stream;
-    FFT(f, cufftSetStream(f->c2r, f->stream));
+    if (f->have_c2r) FFT(f, cufftSetStream(f->c2r, f->stream));
     FFT(f, cufftSetStream(f->r2c, f->stream));
     return 0;
 }
@@ -635,12 +856,15 @@ extern "C" int dl_flow_set_velocity(dl_flow *f, const double *u, int64_t pitch_y
         FCUDA(f, cudaMemcpyAsync(tmp, u, sizeof(double) * 3 * comp, cudaMemcpyHostToDevice, f->stream));
         src = tmp;
     }
+    // packed where the state goes (3 n^3 doubles fit its 3 M modes): the last step's velocity
+    // stays in place, and the state is rewritten from the transform in work
+    double *packed = reinterpret_cast<double *>(f->u);
     for (int c = 0; c < 3; c++) {
-        k_pack<<<blocks(n3, 256), 256, 0, f->stream>>>(n, src + c * comp, pitch_y, pitch_z, f->phys + c * n3);
+        k_pack<<<blocks(n3, 256), 256, 0, f->stream>>>(n, src + c * comp, pitch_y, pitch_z, packed + c * n3);
         FCUDA(f, cudaGetLastError());
     }
     if (tmp) FCUDA(f, cudaFreeAsync(tmp, f->stream));
-    FFT(f, cufftExecD2Z(f->r2c, f->phys, reinterpret_cast<cufftDoubleComplex *>(f->work)));
+    FFT(f, cufftExecD2Z(f->r2c, packed, reinterpret_cast<cufftDoubleComplex *>(f->work)));
     k_project_scaled<<<blocks(f->G.M, 256), 256, 0, f->stream>>>(f->G, f->work, 1.0 / (double)n3, f->u);
     FCUDA(f, cudaGetLastError());
     int r = finish(f);
@@ -650,6 +874,7 @@ extern "C" int dl_flow_set_velocity(dl_flow *f, const double *u, int64_t pitch_y
     FCUDA(f, cudaStreamSynchronize(f->stream));
     f->state_set = 1;
     f->phys_valid = 0;
+    f->nold_dirty = 0;
     return 0;
 }
 
@@ -658,24 +883,29 @@ extern "C" int dl_flow_set_spectral(dl_flow *f, const double *uh, const double *
     if (!f || !uh) return DL_E_ARG;
     const cudaMemcpyKind k = on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
     const size_t bytes = sizeof(double2) * 3 * f->G.M;
-    FCUDA(f, cudaMemcpyAsync(f->u, uh, bytes, k, f->stream));
-    int r = finish(f);
+    int r = copy_state(f, f->u, const_cast<double *>(uh), true, k);
     if (r) return r;
-    if (nold) FCUDA(f, cudaMemcpyAsync(f->nold, nold, bytes, k, f->stream));
-    else FCUDA(f, cudaMemcpyAsync(f->nold, f->u, bytes, cudaMemcpyDeviceToDevice, f->stream));
+    r = finish(f);
+    if (r) return r;
+    if (nold) {
+        r = copy_state(f, f->nold, const_cast<double *>(nold), true, k);
+        if (r) return r;
+    } else FCUDA(f, cudaMemcpyAsync(f->nold, f->u, bytes, cudaMemcpyDeviceToDevice, f->stream));
     FCUDA(f, cudaStreamSynchronize(f->stream));
     f->state_set = 1;
     f->phys_valid = 0;
+    f->nold_dirty = nold != nullptr;
     return 0;
 }
 
 extern "C" int dl_flow_get_spectral(dl_flow *f, double *uh, double *nold)
 {
     if (!f) return DL_E_ARG;
+    if (uh)
+        if (const int r = copy_state(f, f->u, uh, false, cudaMemcpyDeviceToHost)) return r;
+    if (nold)
+        if (const int r = copy_state(f, f->nold, nold, false, cudaMemcpyDeviceToHost)) return r;
     FCUDA(f, cudaStreamSynchronize(f->stream));
-    const size_t bytes = sizeof(double2) * 3 * f->G.M;
-    if (uh) FCUDA(f, cudaMemcpy(uh, f->u, bytes, cudaMemcpyDeviceToHost));
-    if (nold) FCUDA(f, cudaMemcpy(nold, f->nold, bytes, cudaMemcpyDeviceToHost));
     return 0;
 }
 
@@ -715,13 +945,77 @@ extern "C" int dl_flow_step(dl_flow *f, dl_ctx *droplets)
         if (droplets->dc.n != n) return ffail(f, DL_E_ARG, "dl_flow_step: droplet grid differs from the flow's");
         const int r = dl_field_target(droplets, &fpad, &fpy, &fpz, &fpc, &f32);
         if (r) return ffail(f, r, std::string("dl_flow_step: ") + dl_last_error(droplets));
-        // the droplet work queued so far (the last step's interpolation reads the padded
-        // field) completes before this step writes it
+    }
+    // the droplet work queued so far (the last step's interpolation reads the padded field)
+    // completes before this step writes it
+    auto wait_used = [&]() {
+        if (!droplets) return 0;
         FCUDA(f, cudaEventRecord(f->ev_used, droplets->stream));
         FCUDA(f, cudaStreamWaitEvent(f->stream, f->ev_used, 0));
+        return 0;
+    };
+    auto field_ready = [&]() {
+        if (!droplets) return 0;
+        FCUDA(f, cudaEventRecord(f->ev_ready, f->stream));
+        FCUDA(f, cudaStreamWaitEvent(droplets->stream, f->ev_ready, 0));
+        const double *u[3] = {f->vel, f->vel + n3, f->vel + 2 * n3};
+        dl_field_written(droplets, u, n, (int64_t)n * n);
+        return 0;
+    };
+    const double *afor = nullptr;
+    if (f->p.forcing == 2) {
+        double a[450];
+        stochastic_amplitudes(f, a);
+        FCUDA(f, cudaMemcpyAsync(f->afor, a, sizeof(a), cudaMemcpyHostToDevice, f->stream));
+        afor = f->afor;
     }
     cudaEvent_t *te = f->timing ? f->tse + 5 * (f->nts % dl_flow::NTS) : nullptr;
     if (te) FCUDA(f, cudaEventRecord(te[0], f->stream));
+    if (f->fast) {
+        // events: before, after the y transforms of curl u and u (transformed along z by the step
+        // before), after the x pass, after the y and z transforms of N, after the update and the
+        // next step's z transforms
+        XArgs X = x_args(f);
+        X.fp = fpad;
+        X.fpy = fpy;
+        X.fpz = fpz;
+        X.fpc = fpc;
+        with_passes(n, [&](auto P) { P.ypass(f, true); });
+        if (te) FCUDA(f, cudaEventRecord(te[1], f->stream));
+        if (const int r = wait_used()) return r;
+        with_passes(n, [&](auto P) { P.xpass(f, !droplets ? X_STEP : (f32 ? X_EMIT32 : X_EMIT64), X); });
+        FCUDA(f, cudaGetLastError());
+        if (const int r = field_ready()) return r;
+        if (te) FCUDA(f, cudaEventRecord(te[2], f->stream));
+        f->phys_valid = 1;
+        if (f->nold_dirty) {
+            k_dealias<<<blocks(f->G.M, 256), 256, 0, f->stream>>>(f->G, f->nold);
+            FCUDA(f, cudaGetLastError());
+            f->nold_dirty = 0;
+        }
+        ZArgs Z = z_args(f);
+        Z.afor = afor;
+        Z.det = f->p.forcing == 1;
+        Z.f1 = f->p.force[0];
+        Z.f2 = f->p.force[1];
+        with_passes(n, [&](auto P) {
+            P.ypass(f, false);
+            P.zforward(f, Z);
+        });
+        if (te) FCUDA(f, cudaEventRecord(te[3], f->stream));
+        k_update_sphere<<<blocks((int64_t)n * n * (n / 2), 256), 256, 0, f->stream>>>(Z);
+        k_low<<<blocks((int64_t)n * n, 128), 128, 0, f->stream>>>(Z);
+        with_passes(n, [&](auto P) { P.zinverse(f, Z, false); });
+        FCUDA(f, cudaGetLastError());
+        if (te) {
+            FCUDA(f, cudaEventRecord(te[4], f->stream));
+            f->nts++;
+        }
+        f->launches += 7;
+        f->steps++;
+        return 0;
+    }
+    if (const int r = wait_used()) return r;
     // omega and u in physical space
     FFT(f, cufftExecZ2D(f->c2r, reinterpret_cast<cufftDoubleComplex *>(f->work), f->phys));
     if (te) FCUDA(f, cudaEventRecord(te[1], f->stream));
@@ -734,10 +1028,7 @@ extern "C" int dl_flow_step(dl_flow *f, dl_ctx *droplets)
         else
             k_cross_emit<double><<<grid, 128, 0, f->stream>>>(n, f->phys, (double *)fpad, fpy, fpz, fpc);
         FCUDA(f, cudaGetLastError());
-        FCUDA(f, cudaEventRecord(f->ev_ready, f->stream));
-        FCUDA(f, cudaStreamWaitEvent(droplets->stream, f->ev_ready, 0));
-        const double *u[3] = {f->phys + 3 * n3, f->phys + 4 * n3, f->phys + 5 * n3};
-        dl_field_written(droplets, u, n, (int64_t)n * n);
+        if (const int r = field_ready()) return r;
     } else {
         k_cross<<<blocks(n3, 256), 256, 0, f->stream>>>(n3, f->phys);
         FCUDA(f, cudaGetLastError());
@@ -753,15 +1044,9 @@ extern "C" int dl_flow_step(dl_flow *f, dl_ctx *droplets)
     A.nu = f->p.nu;
     A.dt = f->p.dt;
     A.inv_n3 = 1.0 / (double)n3;
-    A.afor = nullptr;
+    A.afor = afor;
     A.work = f->work;
     A.emit = 1;
-    if (f->p.forcing == 2) {
-        double a[450];
-        stochastic_amplitudes(f, a);
-        FCUDA(f, cudaMemcpyAsync(f->afor, a, sizeof(a), cudaMemcpyHostToDevice, f->stream));
-        A.afor = f->afor;
-    }
     k_update<<<blocks(f->G.M, 256), 256, 0, f->stream>>>(A);
     FCUDA(f, cudaGetLastError());
     if (f->p.forcing == 1) {
@@ -806,7 +1091,7 @@ extern "C" int dl_flow_timing(dl_flow *f, int enable, double *ms4, int *steps)
 extern "C" const double *dl_flow_velocity(dl_flow *f, int icpt)
 {
     if (!f || icpt < 1 || icpt > 3 || !f->phys_valid) return nullptr;
-    return f->phys + (int64_t)(2 + icpt) * f->G.n * f->G.n * f->G.n;
+    return f->vel + (int64_t)(icpt - 1) * f->G.n * f->G.n * f->G.n;
 }
 
 extern "C" int dl_flow_dissipation(dl_flow *f, const double **field)
@@ -816,6 +1101,26 @@ extern "C" int dl_flow_dissipation(dl_flow *f, const double **field)
     if (!f->state_set) return ffail(f, DL_E_STATE, "dl_flow_dissipation: set the velocity first");
     const int n = f->G.n;
     const int64_t n3 = (int64_t)n * n * n;
+    if (f->fast) {
+        if (!f->diss && cudaMalloc(&f->diss, sizeof(double) * n3) != cudaSuccess)
+            return ffail(f, DL_E_ALLOC, "dl_flow_dissipation: buffers");
+        // the strain takes W's place, which is then transformed from the state again
+        int r = transform_state(f, true);
+        if (r) return r;
+        XArgs X = x_args(f);
+        X.diss = f->diss;
+        X.nu2 = 2.0 * f->p.nu;
+        with_passes(n, [&](auto P) {
+            P.ypass(f, true);
+            P.xpass(f, X_DISS, X);
+        });
+        f->launches += 2;
+        FCUDA(f, cudaGetLastError());
+        r = transform_state(f, false);
+        if (r) return r;
+        *field = f->diss;
+        return 0;
+    }
     if (!f->diss) {
         if (cudaMalloc(&f->diss_spec, sizeof(double2) * f->G.M) != cudaSuccess ||
             cudaMalloc(&f->diss_phys, sizeof(double) * n3) != cudaSuccess ||

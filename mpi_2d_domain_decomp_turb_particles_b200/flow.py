@@ -128,8 +128,8 @@ class Flow:
 
     def timing(self, enable: bool = True):
         """Device ms per step averaged over the steps since the last call: a dict with the
-        inverse transform, cross-product kernel, forward transform and update kernels, and
-        the step count; then enables or disables the timing for the steps that follow."""
+        inverse transform, cross-product kernel, forward transform and update kernels (as
+        dl_flow_timing divides them), and the step count; then enables or disables the timing for the steps that follow."""
         ms = (C.c_double * 4)()
         n = C.c_int(0)
         self._chk(self.lib.dl_flow_timing(self.h, int(enable), ms, C.byref(n)))
