@@ -113,7 +113,7 @@ __global__ void k_upload(int nps, const double *yp, const double *fvp, const dou
 
 template <typename T>
 struct DownArgs {
-    int nps;
+    int r0, r1;           // reference indices of this launch; the outputs start at r0
     const int *dev_of_ref;
     const double *px, *py, *pz, *rad, *gid;
     const T *yv[3];       // yp(4:6)
@@ -126,9 +126,9 @@ struct DownArgs {
 template <typename T>
 __global__ void k_download(DownArgs<T> A)
 {
-    int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= A.nps) return;
-    int d = A.dev_of_ref[r];
+    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= A.r1 - A.r0) return;
+    const int d = A.dev_of_ref[A.r0 + r];
     if (A.yp) {
         double *y = A.yp + (int64_t)r * 8;
         y[0] = A.px[d]; y[1] = A.py[d]; y[2] = A.pz[d];
@@ -458,7 +458,8 @@ static int allocate_state(dl_ctx *c)
     ALLOC(c->lv_dep, sizeof(int) * m);
     ALLOC(c->d_err, sizeof(int));
     ALLOC(c->col_work, 2 * sizeof(int));
-    ALLOC(c->xfer64, sizeof(double) * (3 * m + 16));
+    c->xfer_cap = std::max<size_t>(3 * (size_t)m + 16, 1 << 20);
+    ALLOC(c->xfer64, sizeof(double) * c->xfer_cap);
     ALLOC(c->xfer_i, sizeof(int) * (4 * m + 16));
     // statistics
     c->nbinsz = c->dc.nset * c->dc.nset * DL_NBIN;
@@ -750,12 +751,9 @@ static int download_t(dl_ctx *c, double *yp, double *fvp, double *fdp, double *v
 {
     const int nps = c->nps;
     if (nps == 0) return 0;
-    size_t n8 = (yp ? 8 : 0) + (fvp ? 9 : 0) + (fdp ? 12 : 0) + (vp ? 3 : 0) + (dm ? 3 : 0);
-    double *buf = nullptr;
-    DL_CUDA(c, cudaMallocAsync((void **)&buf, (size_t)nps * n8 * 8 + 8, c->stream));
+    const size_t n8 = (yp ? 8 : 0) + (fvp ? 9 : 0) + (fdp ? 12 : 0) + (vp ? 3 : 0) + (dm ? 3 : 0);
     DownArgs<T> A;
     memset(&A, 0, sizeof(A));
-    A.nps = nps;
     A.dev_of_ref = c->dev_of_ref;
     A.px = c->pos[c->pcur][0]; A.py = c->pos[c->pcur][1]; A.pz = c->pos[c->pcur][2];
     A.rad = c->rad; A.gid = c->gid;
@@ -782,20 +780,29 @@ static int download_t(dl_ctx *c, double *yp, double *fvp, double *fdp, double *v
         A.vp[k] = tp<T>(dl_vp_ptr(c, k));
         A.dm[k] = tp<T>(c->dmv[k]);
     }
-    double *q = buf;
-    if (yp) { A.yp = q; q += (size_t)nps * 8; }
-    if (fvp) { A.fvp = q; q += (size_t)nps * 9; }
-    if (fdp) { A.fdp = q; q += (size_t)nps * 12; }
-    if (vp) { A.vpo = q; q += (size_t)nps * 3; }
-    if (dm) { A.dmo = q; q += (size_t)nps * 3; }
-    k_download<T><<<dl_blocks(nps, 256), 256, 0, c->stream>>>(A);
-    DL_CHECK_LAUNCH(c);
-    if (yp) DL_CUDA(c, cudaMemcpyAsync(yp, A.yp, (size_t)nps * 8 * 8, cudaMemcpyDeviceToHost, c->stream));
-    if (fvp) DL_CUDA(c, cudaMemcpyAsync(fvp, A.fvp, (size_t)nps * 9 * 8, cudaMemcpyDeviceToHost, c->stream));
-    if (fdp) DL_CUDA(c, cudaMemcpyAsync(fdp, A.fdp, (size_t)nps * 12 * 8, cudaMemcpyDeviceToHost, c->stream));
-    if (vp) DL_CUDA(c, cudaMemcpyAsync(vp, A.vpo, (size_t)nps * 3 * 8, cudaMemcpyDeviceToHost, c->stream));
-    if (dm) DL_CUDA(c, cudaMemcpyAsync(dm, A.dmo, (size_t)nps * 3 * 8, cudaMemcpyDeviceToHost, c->stream));
-    DL_CUDA(c, cudaFreeAsync(buf, c->stream));
+    // packed and copied in pieces through the context's transfer buffer: a buffer of the whole
+    // size from the stream-ordered allocator is mapped anew on every call, since each
+    // synchronisation gives its pool back (0.3 ms at 20,000 droplets, 0.7-1.0 ms at 1M)
+    const int rows = n8 ? (int)std::min<size_t>(nps, c->xfer_cap / n8) : 0;
+    for (int r0 = 0; rows > 0 && r0 < nps; r0 += rows) {
+        A.r0 = r0;
+        A.r1 = std::min(nps, r0 + rows);
+        const size_t m = A.r1 - r0;
+        const struct { double *host, **dev; int w; } part[5] = {
+            {yp, &A.yp, 8}, {fvp, &A.fvp, 9}, {fdp, &A.fdp, 12}, {vp, &A.vpo, 3}, {dm, &A.dmo, 3}};
+        double *q = c->xfer64;
+        for (const auto &x : part)
+            if (x.host) {
+                *x.dev = q;
+                q += m * x.w;
+            }
+        k_download<T><<<dl_blocks(m, 256), 256, 0, c->stream>>>(A);
+        DL_CHECK_LAUNCH(c);
+        for (const auto &x : part)
+            if (x.host)
+                DL_CUDA(c, cudaMemcpyAsync(x.host + (size_t)r0 * x.w, *x.dev, m * x.w * 8, cudaMemcpyDeviceToHost,
+                                           c->stream));
+    }
     DL_CUDA(c, cudaStreamSynchronize(c->stream));
     return 0;
 }
@@ -813,14 +820,12 @@ static int pert_io_t(dl_ctx *c, double *host, int dir)
 {
     const int nps = c->nps;
     if (nps == 0) return 0;
-    double *buf = nullptr;
-    DL_CUDA(c, cudaMallocAsync((void **)&buf, (size_t)nps * 3 * 8, c->stream));
+    double *buf = c->xfer64;   // holds 3 * msize
     if (dir) DL_CUDA(c, cudaMemcpyAsync(buf, host, (size_t)nps * 24, cudaMemcpyHostToDevice, c->stream));
     k_pert_io<T><<<dl_blocks(nps, 256), 256, 0, c->stream>>>(nps, c->dev_of_ref, tp<T>(c->pert[0]), tp<T>(c->pert[1]),
                                                             tp<T>(c->pert[2]), buf, dir);
     DL_CHECK_LAUNCH(c);
     if (!dir) DL_CUDA(c, cudaMemcpyAsync(host, buf, (size_t)nps * 24, cudaMemcpyDeviceToHost, c->stream));
-    DL_CUDA(c, cudaFreeAsync(buf, c->stream));
     DL_CUDA(c, cudaStreamSynchronize(c->stream));
     return 0;
 }

@@ -757,6 +757,95 @@ __global__ void k_adj_finish(int np, double cd, const double *xbar, const double
 }  // namespace
 
 // ---------------------------------------------------------------------------------------
+// Internal droplet order: a stable radix sort by the Morton code of the cell of the initial
+// position, 8 bits per pass (one counting pass, a scan over (digit, block), one scatter).
+// On the device, because the host's stable sort with the copies around it took 20 of the 44 ms
+// of a 200,000 droplet, 100 step loss and gradient; 0.13 ms here, and the same order.
+// ---------------------------------------------------------------------------------------
+__device__ __forceinline__ unsigned long long spread3(unsigned long long v)
+{
+    v &= 0x1fffff;
+    v = (v | v << 32) & 0x1f00000000ffffULL;
+    v = (v | v << 16) & 0x1f0000ff0000ffULL;
+    v = (v | v << 8) & 0x100f00f00f00f00fULL;
+    v = (v | v << 4) & 0x10c30c30c30c30c3ULL;
+    v = (v | v << 2) & 0x1249249249249249ULL;
+    return v;
+}
+
+__global__ void k_adj_keys(int np, int n, double pi2, double dx, const double *x, unsigned long long *key, int *order)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= np) return;
+    unsigned long long c[3];
+    for (int d = 0; d < 3; d++) {
+        const double v = x[3 * (int64_t)i + d], w = v - pi2 * floor(v / pi2);
+        c[d] = (unsigned long long)min(max((int)(w / dx), 0), n - 1);
+    }
+    key[i] = spread3(c[0]) | spread3(c[1]) << 1 | spread3(c[2]) << 2;
+    order[i] = i;
+}
+
+constexpr int kSortBlock = 256;   // keys per block, one per thread
+
+__global__ void __launch_bounds__(kSortBlock) k_adj_digits(int np, const unsigned long long *key, int shift, int nblk,
+                                                           int *cnt)
+{
+    __shared__ int c[256];
+    c[threadIdx.x] = 0;
+    __syncthreads();
+    const int i = blockIdx.x * kSortBlock + threadIdx.x;
+    if (i < np) atomicAdd(&c[(int)(key[i] >> shift) & 255], 1);
+    __syncthreads();
+    cnt[threadIdx.x * nblk + blockIdx.x] = c[threadIdx.x];
+}
+
+// stable within the block: rank = equal digits in earlier warps and in lower lanes
+__global__ void __launch_bounds__(kSortBlock) k_adj_radix(int np, const unsigned long long *key, const int *order,
+                                                          int shift, int nblk, const int *start,
+                                                          unsigned long long *key_out, int *order_out)
+{
+    __shared__ int c[kSortBlock / 32][256];
+    const int i = blockIdx.x * kSortBlock + threadIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (int q = 0; q < kSortBlock / 32; q++) c[q][threadIdx.x] = 0;
+    __syncthreads();
+    const unsigned long long k = i < np ? key[i] : 0;
+    const int d = i < np ? (int)(k >> shift) & 255 : -1;
+    const unsigned same = __match_any_sync(0xffffffffu, d);
+    const int rank = __popc(same & ((1u << lane) - 1));
+    if (d >= 0 && rank == 0) c[w][d] = __popc(same);
+    __syncthreads();
+    if (d < 0) return;
+    int at = start[d * nblk + blockIdx.x] + rank;
+    for (int q = 0; q < w; q++) at += c[q][d];
+    key_out[at] = k;
+    order_out[at] = order[i];
+}
+
+// droplets in the internal order
+__global__ void k_adj_reorder(int np, const int *order, const double *x, const double *tau, const double *rad,
+                              double *xo, double *to, double *ro)
+{
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= np) return;
+    const int64_t i = order[q];
+    for (int d = 0; d < 3; d++) xo[3 * (int64_t)q + d] = x[3 * i + d];
+    to[q] = tau[i];
+    ro[q] = rad[i];
+}
+
+// pairs with the droplet first in the caller's order first, and their caller's indices
+__global__ void k_adj_pair_refs(int m, const int *perm, int2 *pairs, int2 *refs)
+{
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= m) return;
+    int2 p = pairs[q];
+    if (perm[p.x] > perm[p.y]) p = make_int2(p.y, p.x);
+    pairs[q] = p;
+    refs[q] = make_int2(perm[p.x], perm[p.y]);
+}
+
+// ---------------------------------------------------------------------------------------
 // Context
 // ---------------------------------------------------------------------------------------
 struct dl_adj {
@@ -783,8 +872,11 @@ struct dl_adj {
     int *cell_cnt = nullptr, *cell_start = nullptr, *cell_fill = nullptr, *cell_key = nullptr, *cell_order = nullptr;
     int *scan_tmp = nullptr;
     int *perm = nullptr;          // internal droplet index -> caller's index
-    std::vector<int> hperm;
-    int2 *pairs = nullptr;
+    unsigned long long *sort_key[2] = {nullptr, nullptr};
+    int *sort_order = nullptr;    // the other buffer of perm while sorting
+    int *sort_cnt = nullptr, *sort_start = nullptr, *sort_scan = nullptr;
+    double *rmax = nullptr;
+    int2 *pairs = nullptr, *pair_refs = nullptr;
     int *d_npairs = nullptr;
     int npairs = 0, pair_cap = 0, nc = 0;
     double *red = nullptr;   // partials + outputs + ticket
@@ -935,9 +1027,11 @@ int find_pairs(dl_adj *a)
     ACUDA(a, cudaStreamSynchronize(a->stream));
     if (np2 > a->pair_cap) {
         cudaFree(a->pairs);
-        a->pairs = nullptr;
+        cudaFree(a->pair_refs);
+        a->pairs = a->pair_refs = nullptr;
         a->pair_cap = np2 + np2 / 4 + 1024;
-        const int ra = aalloc(a, (void **)&a->pairs, sizeof(int2) * a->pair_cap);
+        int ra = aalloc(a, (void **)&a->pairs, sizeof(int2) * a->pair_cap);
+        if (!ra) ra = aalloc(a, (void **)&a->pair_refs, sizeof(int2) * a->pair_cap);
         if (ra) return ra;
         return find_pairs<T>(a);
     }
@@ -945,14 +1039,19 @@ int find_pairs(dl_adj *a)
     if (np2 > 0) {
         // (i, j) with i before j in the caller's order, sorted by the caller's indices: the
         // pair sum then runs in the order of the reference's (i, j > i) loops
-        const std::vector<int> &pm = a->hperm;
-        std::vector<int2> h(np2);
-        ACUDA(a, cudaMemcpy(h.data(), a->pairs, sizeof(int2) * np2, cudaMemcpyDeviceToHost));
-        for (auto &q : h)
-            if (pm[q.x] > pm[q.y]) std::swap(q.x, q.y);
-        std::sort(h.begin(), h.end(), [&](const int2 &u, const int2 &v) {
-            return pm[u.x] != pm[v.x] ? pm[u.x] < pm[v.x] : pm[u.y] < pm[v.y];
+        k_adj_pair_refs<<<dl_blocks(np2, 128), 128, 0, a->stream>>>(np2, a->perm, a->pairs, a->pair_refs);
+        ACUDA(a, cudaGetLastError());
+        std::vector<int2> h(np2), ref(np2);
+        ACUDA(a, cudaMemcpyAsync(h.data(), a->pairs, sizeof(int2) * np2, cudaMemcpyDeviceToHost, a->stream));
+        ACUDA(a, cudaMemcpyAsync(ref.data(), a->pair_refs, sizeof(int2) * np2, cudaMemcpyDeviceToHost, a->stream));
+        ACUDA(a, cudaStreamSynchronize(a->stream));
+        std::vector<int> ord(np2);
+        for (int q = 0; q < np2; q++) ord[q] = q;
+        std::sort(ord.begin(), ord.end(), [&](int u, int v) {
+            return ref[u].x != ref[v].x ? ref[u].x < ref[v].x : ref[u].y < ref[v].y;
         });
+        for (int q = 0; q < np2; q++) ref[q] = h[ord[q]];
+        h.swap(ref);
         ACUDA(a, cudaMemcpyAsync(a->pairs, h.data(), sizeof(int2) * np2, cudaMemcpyHostToDevice, a->stream));
     }
     return 0;
@@ -1109,6 +1208,15 @@ extern "C" int dl_adj_create(const dl_adj_params *p, dl_adj **out)
     ADJ_ALLOC(a->perm, sizeof(int) * np);
     ADJ_ALLOC(a->cell_order, sizeof(int) * np);
     ADJ_ALLOC(a->pairs, sizeof(int2) * a->pair_cap);
+    ADJ_ALLOC(a->pair_refs, sizeof(int2) * a->pair_cap);
+    const size_t ncnt = 256 * (size_t)dl_blocks((long)np, kSortBlock);
+    ADJ_ALLOC(a->sort_key[0], 8 * np);
+    ADJ_ALLOC(a->sort_key[1], 8 * np);
+    ADJ_ALLOC(a->sort_order, sizeof(int) * np);
+    ADJ_ALLOC(a->sort_cnt, sizeof(int) * ncnt);
+    ADJ_ALLOC(a->sort_start, sizeof(int) * (ncnt + 1));
+    ADJ_ALLOC(a->sort_scan, sizeof(int) * 2 * (ncnt / 1024 + 4));
+    ADJ_ALLOC(a->rmax, sizeof(double));
     ADJ_ALLOC(a->d_npairs, sizeof(int));
     ADJ_ALLOC(a->red, sizeof(double) * 544);
 #undef ADJ_ALLOC
@@ -1132,7 +1240,8 @@ extern "C" int dl_adj_destroy(dl_adj *a)
     if (a->own_stream) cudaStreamSynchronize(a->own_stream);
     void *ptrs[] = {a->fpad, a->gpad, a->x0, a->tau, a->rad, a->xs, a->ss, a->ckx, a->cks, a->TX, a->TV, a->TU, a->TJ,
                     a->xbar, a->taubar, a->P, a->Q, a->cell_cnt, a->cell_start, a->cell_fill, a->scan_tmp,
-                    a->cell_key, a->cell_order, a->pairs, a->d_npairs, a->red, a->perm};
+                    a->cell_key, a->cell_order, a->pairs, a->d_npairs, a->red, a->perm, a->pair_refs,
+                    a->sort_key[0], a->sort_key[1], a->sort_order, a->sort_cnt, a->sort_start, a->sort_scan, a->rmax};
     for (void *q : ptrs)
         if (q) cudaFree(q);
     for (auto &e : a->ev)
@@ -1186,52 +1295,45 @@ extern "C" int dl_adj_set_field(dl_adj *a, int icpt, const double *v, int64_t pi
 extern "C" int dl_adj_set_droplets(dl_adj *a, const double *x0, const double *tau, const double *radius, int on_device)
 {
     if (!a || !x0 || !tau || !radius) return DL_E_ARG;
-    const size_t np = a->p.np;
-    std::vector<double> hx(3 * np), ht(np), hr(np);
-    const cudaMemcpyKind k = on_device ? cudaMemcpyDeviceToHost : cudaMemcpyHostToHost;
-    ACUDA(a, cudaStreamSynchronize(a->stream));
-    ACUDA(a, cudaMemcpy(hx.data(), x0, sizeof(double) * 3 * np, k));
-    ACUDA(a, cudaMemcpy(ht.data(), tau, sizeof(double) * np, k));
-    ACUDA(a, cudaMemcpy(hr.data(), radius, sizeof(double) * np, k));
+    const int np = a->p.np;
+    const double *dx = x0, *dtau = tau, *drad = radius;
+    double *tmp = nullptr;
+    if (!on_device) {
+        ACUDA(a, cudaMallocAsync((void **)&tmp, sizeof(double) * 5 * (size_t)np, a->stream));
+        const size_t b = sizeof(double) * (size_t)np;
+        ACUDA(a, cudaMemcpyAsync(tmp, x0, 3 * b, cudaMemcpyHostToDevice, a->stream));
+        ACUDA(a, cudaMemcpyAsync(tmp + 3 * (size_t)np, tau, b, cudaMemcpyHostToDevice, a->stream));
+        ACUDA(a, cudaMemcpyAsync(tmp + 4 * (size_t)np, radius, b, cudaMemcpyHostToDevice, a->stream));
+        dx = tmp;
+        dtau = tmp + 3 * (size_t)np;
+        drad = tmp + 4 * (size_t)np;
+    }
     // internal order: droplets sorted along the Morton curve of the cells of their initial
     // position, so that the stencils of a warp cover a compact box (shared cache lines in
     // the gathers, nearby grid points in the gradient atomics)
-    auto spread = [](uint64_t v) {
-        v &= 0x1fffff;
-        v = (v | v << 32) & 0x1f00000000ffffULL;
-        v = (v | v << 16) & 0x1f0000ff0000ffULL;
-        v = (v | v << 8) & 0x100f00f00f00f00fULL;
-        v = (v | v << 4) & 0x10c30c30c30c30c3ULL;
-        v = (v | v << 2) & 0x1249249249249249ULL;
-        return v;
-    };
-    std::vector<uint64_t> key(np);
-    for (size_t i = 0; i < np; i++) {
-        uint64_t c[3];
-        for (int d = 0; d < 3; d++) {
-            const double w = hx[3 * i + d] - a->pi2 * std::floor(hx[3 * i + d] / a->pi2);
-            const int q = (int)(w / a->dx);
-            c[d] = (uint64_t)std::min(std::max(q, 0), a->n - 1);
-        }
-        key[i] = spread(c[0]) | spread(c[1]) << 1 | spread(c[2]) << 2;
+    int bits = 0;   // per direction; the code has 3 * bits
+    while (bits < 21 && (1 << bits) < a->n) bits++;
+    const int passes = (3 * bits + 7) / 8, nblk = dl_blocks(np, kSortBlock);
+    int *order[2] = {a->perm, a->sort_order};
+    int cur = passes & 1;   // the last pass writes perm
+    k_adj_keys<<<dl_blocks(np, 256), 256, 0, a->stream>>>(np, a->n, a->pi2, a->dx, dx, a->sort_key[cur], order[cur]);
+    ACUDA(a, cudaGetLastError());
+    for (int p = 0; p < passes; p++, cur ^= 1) {
+        k_adj_digits<<<nblk, kSortBlock, 0, a->stream>>>(np, a->sort_key[cur], 8 * p, nblk, a->sort_cnt);
+        ACUDA(a, dl_scan_counts(a->stream, a->sort_cnt, a->sort_start, 256 * nblk, a->sort_scan, nullptr));
+        k_adj_radix<<<nblk, kSortBlock, 0, a->stream>>>(np, a->sort_key[cur], order[cur], 8 * p, nblk, a->sort_start,
+                                                        a->sort_key[cur ^ 1], order[cur ^ 1]);
+        ACUDA(a, cudaGetLastError());
     }
-    std::vector<int> order(np);
-    for (size_t i = 0; i < np; i++) order[i] = (int)i;
-    std::stable_sort(order.begin(), order.end(), [&](int u, int v) { return key[u] < key[v]; });
-    a->hperm = order;   // internal index -> caller's index
-    std::vector<double> sx(3 * np), st(np), sr(np);
-    for (size_t q = 0; q < np; q++) {
-        const int i = order[q];
-        for (int d = 0; d < 3; d++) sx[3 * q + d] = hx[3 * (size_t)i + d];
-        st[q] = ht[i];
-        sr[q] = hr[i];
-    }
-    ACUDA(a, cudaMemcpyAsync(a->x0, sx.data(), sizeof(double) * 3 * np, cudaMemcpyHostToDevice, a->stream));
-    ACUDA(a, cudaMemcpyAsync(a->tau, st.data(), sizeof(double) * np, cudaMemcpyHostToDevice, a->stream));
-    ACUDA(a, cudaMemcpyAsync(a->rad, sr.data(), sizeof(double) * np, cudaMemcpyHostToDevice, a->stream));
-    ACUDA(a, cudaMemcpyAsync(a->perm, order.data(), sizeof(int) * np, cudaMemcpyHostToDevice, a->stream));
+    k_adj_reorder<<<dl_blocks(np, 256), 256, 0, a->stream>>>(np, a->perm, dx, dtau, drad, a->x0, a->tau, a->rad);
+    ACUDA(a, cudaMemsetAsync(a->rmax, 0, sizeof(double), a->stream));
+    k_rad_max<<<std::min(296, dl_blocks(np, 256)), 256, 0, a->stream>>>(np, a->rad, (unsigned long long *)a->rmax);
+    ACUDA(a, cudaGetLastError());
+    if (tmp) ACUDA(a, cudaFreeAsync(tmp, a->stream));
+    double rmax = 0.0;
+    ACUDA(a, cudaMemcpyAsync(&rmax, a->rmax, sizeof(double), cudaMemcpyDeviceToHost, a->stream));
+    ACUDA(a, cudaStreamSynchronize(a->stream));
     // pair cells at least as wide as the largest cutoff
-    const double rmax = *std::max_element(hr.begin(), hr.end());
     const double cut = a->p.pair_factor * 2.0 * rmax;
     int nc = cut > 0.0 ? (int)std::floor(a->pi2 / cut) : 128;
     a->nc = std::max(3, std::min(128, nc));
@@ -1267,7 +1369,8 @@ extern "C" int dl_adj_get_final(dl_adj *a, double *xN, double *vN)
     std::vector<double> x(3 * (size_t)np);
     ACUDA(a, cudaStreamSynchronize(a->stream));
     ACUDA(a, cudaMemcpy(x.data(), a->xs, sizeof(double) * 3 * np, cudaMemcpyDeviceToHost));
-    const std::vector<int> &pm = a->hperm;
+    std::vector<int> pm(np);
+    ACUDA(a, cudaMemcpy(pm.data(), a->perm, sizeof(int) * np, cudaMemcpyDeviceToHost));
     if (xN)
         for (int i = 0; i < np; i++)
             for (int c = 0; c < 3; c++) xN[3 * pm[i] + c] = x[(size_t)c * np + i];

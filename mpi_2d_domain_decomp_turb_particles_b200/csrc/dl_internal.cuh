@@ -164,7 +164,8 @@ struct dl_ctx {
     int *lv_src;                 // [msize] (HDI) device holding each new reference index before the reorder
     void *pert_tmp;              // [3 * msize] (HDI) pertvel values kept at their reference index
     int *d_err;                  // device error flags (see DL_DERR_*)
-    double *xfer64;              // [3 * msize] host<->device transfer scratch
+    double *xfer64;              // [xfer_cap >= 3 * msize] host<->device transfer scratch
+    size_t xfer_cap;
     int *xfer_i;                 // [4 * msize] host<->device transfer scratch
 
     // ---- COLLISION_DET outputs ----
