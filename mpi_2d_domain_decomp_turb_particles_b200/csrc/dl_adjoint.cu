@@ -138,73 +138,141 @@ __device__ __forceinline__ void interp(const Field<double> &F, const double *x, 
     }
 }
 
-__device__ __forceinline__ void interp(const Field<float> &F, const double *x, float *out)
-{
-    float b[3][6];
-    const int64_t c0 = stencil_at<float>(F, x, b, nullptr);
-    float acc[3] = {0.0f, 0.0f, 0.0f};
-#pragma unroll
-    for (int c = 0; c < 6; c++) {
-        float tz[3] = {0.0f, 0.0f, 0.0f};
-#pragma unroll
-        for (int bb = 0; bb < 6; bb++) {
-            const float4 *row = reinterpret_cast<const float4 *>(F.f) + c0 + F.pz * c + F.py * bb;
-            float ty[3] = {0.0f, 0.0f, 0.0f};
-#pragma unroll
-            for (int a = 0; a < 6; a++) {
-                const float4 v = row[a];
-                ty[0] = fmaf(v.x, b[0][a], ty[0]);
-                ty[1] = fmaf(v.y, b[0][a], ty[1]);
-                ty[2] = fmaf(v.z, b[0][a], ty[2]);
-            }
-            for (int q = 0; q < 3; q++) tz[q] = fmaf(ty[q], b[1][bb], tz[q]);
-        }
-        for (int q = 0; q < 3; q++) acc[q] = fmaf(tz[q], b[2][c], acc[q]);
-    }
-    for (int q = 0; q < 3; q++) out[q] = acc[q];
-}
+// FP32 interpolant, and with JAC its Jacobian J[q][k] = dU[q]/d(fraction k) (divide by dx for
+// the spatial derivative), of the eight droplets of a warp, gathered by the whole warp: eight
+// lanes take the x nodes of a stencil row (six used, 96 contiguous bytes) and the four groups of
+// eight lanes take four rows, so that a droplet's 36 rows are nine vector loads of four rows
+// each.  With a droplet per lane every load touches up to 32 cache lines, which bounds it.
+// Every group of lanes carries the state of the same eight droplets (32 droplets per warp,
+// each state once, has a serial chain four times as long: 68 us per step of 200,000 droplets).
+// Per step, before (a droplet per lane) and now: 79 -> 50 us forward at 200,000 droplets in
+// 128^3, 12 -> 7 at 20,000 in 64^3, 8.0 -> 2.6 at 500 in 32^3; with the Jacobian 79 -> 80 us at
+// 200,000 (twelve sums per droplet and FP32 issue make up for the loads), the whole backward
+// pass 18 -> 16 us at 20,000 and 12 -> 7 at 500.  Sharing the stores of the recorded
+// trajectory among the lane groups gave nothing.
+// Rows of lane group r: y node r, z nodes 0..5; then y node 4 + (r & 1), z nodes (r >> 1) + 0, 2, 4.
+constexpr int kWarpDrops = 8;
+// floats of a droplet's slab: 0..2 the corner's x, y and z parts (points), 4..9 bz, 10..15 bx,
+// 16..21 by, and with JAC the derivatives alike 20 floats on
+template <bool JAC>
+__host__ __device__ constexpr int slab_floats() { return JAC ? 44 : 24; }
 
-// FP32 interpolant and its Jacobian in one pass over the stencil: U[q] and
-// J[q][k] = dU[q]/d(fraction k) (divide by dx for the spatial derivative)
-__device__ __forceinline__ void interp_jac(const Field<float> &F, const double *x, float *U, float (*J)[3])
+template <bool JAC>
+__device__ __forceinline__ void interp_warp(const Field<float> &F, const double *x, float *U, float (*J)[3], float *slab)
 {
-    float b[3][6], d[3][6];
-    const int64_t c0 = stencil_at<float>(F, x, b, d);
-    float au[3] = {0.0f, 0.0f, 0.0f}, ax[3] = {0.0f, 0.0f, 0.0f}, ay[3] = {0.0f, 0.0f, 0.0f},
-          az[3] = {0.0f, 0.0f, 0.0f};
+    constexpr int W = slab_floats<JAC>(), D = kWarpDrops, B = JAC ? 4 : 8, C = JAC ? 12 : 3;
+    const int lane = threadIdx.x & 31, xl = lane & 7, r = lane >> 3;
+    if (r < 3) {   // lane group r: direction r of droplet xl
+        const double v = r == 0 ? x[0] : (r == 1 ? x[1] : x[2]);
+        const int node = (int)floor(v / F.dx);
+        const float z = (float)((v - (double)node * F.dx) / F.dx);
+        float b[6];
+        w6(z, b);
+        float *w = slab + xl * W;
+        reinterpret_cast<int *>(w)[r] = wrapn(node, F.n) - 2 + DL_PAD_LO;
+        float *o = w + (r == 0 ? 10 : (r == 1 ? 16 : 4));
+#pragma unroll
+        for (int q = 0; q < 3; q++) reinterpret_cast<float2 *>(o)[q] = make_float2(b[2 * q], b[2 * q + 1]);
+        if (JAC) {
+            dw6(z, b);
+#pragma unroll
+            for (int q = 0; q < 3; q++) reinterpret_cast<float2 *>(o + 20)[q] = make_float2(b[2 * q], b[2 * q + 1]);
+        }
+    }
+    __syncwarp();
+    const float4 *base = reinterpret_cast<const float4 *>(F.f) + xl;
+    const int y1 = 4 + (r & 1), zo = r >> 1;
 #pragma unroll 1
-    for (int c = 0; c < 6; c++) {
-        float tu[3] = {0.0f, 0.0f, 0.0f}, tx[3] = {0.0f, 0.0f, 0.0f}, ty[3] = {0.0f, 0.0f, 0.0f};
+    for (int bt = 0; bt < D / B; bt++) {
+        float s[B][C];   // this lane's part of the B droplets' sums
 #pragma unroll
-        for (int bb = 0; bb < 6; bb++) {
-            const float4 *row = reinterpret_cast<const float4 *>(F.f) + c0 + F.pz * c + F.py * bb;
-            float ru[3] = {0.0f, 0.0f, 0.0f}, rx[3] = {0.0f, 0.0f, 0.0f};
+        for (int k = 0; k < B; k++) {
+            const float *w = slab + (bt * B + k) * W;
+            const int4 h = reinterpret_cast<const int4 *>(w)[0];
+            const float4 l = reinterpret_cast<const float4 *>(w)[1];
+            const float2 m = reinterpret_cast<const float2 *>(w)[4];
+            const int64_t c0 = h.x + F.py * h.y + F.pz * h.z;
+            const float bz[6] = {l.x, l.y, l.z, l.w, m.x, m.y};
+            float4 v[9];
+            const float4 *p0 = base + c0 + F.py * r, *p1 = base + c0 + F.py * y1 + F.pz * zo;
 #pragma unroll
-            for (int a = 0; a < 6; a++) {
-                const float4 v = row[a];
-                ru[0] = fmaf(v.x, b[0][a], ru[0]); rx[0] = fmaf(v.x, d[0][a], rx[0]);
-                ru[1] = fmaf(v.y, b[0][a], ru[1]); rx[1] = fmaf(v.y, d[0][a], rx[1]);
-                ru[2] = fmaf(v.z, b[0][a], ru[2]); rx[2] = fmaf(v.z, d[0][a], rx[2]);
+            for (int q = 0; q < 9; q++) {
+                v[q] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                if (xl < 6) v[q] = q < 6 ? p0[F.pz * q] : p1[F.pz * 2 * (q - 6)];
+            }
+            const float bx = w[10 + min(xl, 5)], by0 = w[16 + r], by1 = w[16 + y1];
+            float a0[3] = {0.0f, 0.0f, 0.0f}, a1[3] = {0.0f, 0.0f, 0.0f};
+#pragma unroll
+            for (int q = 0; q < 6; q++) {
+                a0[0] = fmaf(v[q].x, bz[q], a0[0]);
+                a0[1] = fmaf(v[q].y, bz[q], a0[1]);
+                a0[2] = fmaf(v[q].z, bz[q], a0[2]);
             }
 #pragma unroll
+            for (int q = 6; q < 9; q++) {
+                const float wz = zo ? bz[2 * (q - 6) + 1] : bz[2 * (q - 6)];
+                a1[0] = fmaf(v[q].x, wz, a1[0]);
+                a1[1] = fmaf(v[q].y, wz, a1[1]);
+                a1[2] = fmaf(v[q].z, wz, a1[2]);
+            }
+            if constexpr (!JAC) {
+#pragma unroll
+                for (int c = 0; c < 3; c++) s[k][c] = bx * fmaf(a1[c], by1, a0[c] * by0);
+            } else {
+                const float4 ld = reinterpret_cast<const float4 *>(w)[6];
+                const float2 md = reinterpret_cast<const float2 *>(w)[14];
+                const float dz[6] = {ld.x, ld.y, ld.z, ld.w, md.x, md.y};
+                const float dx = w[30 + min(xl, 5)], dy0 = w[36 + r], dy1 = w[36 + y1];
+                float e0[3] = {0.0f, 0.0f, 0.0f}, e1[3] = {0.0f, 0.0f, 0.0f};
+#pragma unroll
+                for (int q = 0; q < 6; q++) {
+                    e0[0] = fmaf(v[q].x, dz[q], e0[0]);
+                    e0[1] = fmaf(v[q].y, dz[q], e0[1]);
+                    e0[2] = fmaf(v[q].z, dz[q], e0[2]);
+                }
+#pragma unroll
+                for (int q = 6; q < 9; q++) {
+                    const float wz = zo ? dz[2 * (q - 6) + 1] : dz[2 * (q - 6)];
+                    e1[0] = fmaf(v[q].x, wz, e1[0]);
+                    e1[1] = fmaf(v[q].y, wz, e1[1]);
+                    e1[2] = fmaf(v[q].z, wz, e1[2]);
+                }
+#pragma unroll
+                for (int c = 0; c < 3; c++) {
+                    const float t = fmaf(a1[c], by1, a0[c] * by0);
+                    s[k][c] = bx * t;
+                    s[k][3 + c] = dx * t;
+                    s[k][6 + c] = bx * fmaf(a1[c], dy1, a0[c] * dy0);
+                    s[k][9 + c] = bx * fmaf(e1[c], by1, e0[c] * by0);
+                }
+            }
+        }
+        // sums over the warp: the first steps halve the droplets a lane still holds, so that
+        // lane l ends with droplet l % B
+#pragma unroll
+        for (int h = B / 2; h > 0; h >>= 1) {
+            const bool up = lane & h;
+#pragma unroll
+            for (int k = 0; k < h; k++)
+#pragma unroll
+                for (int c = 0; c < C; c++) {
+                    const float send = up ? s[k][c] : s[k + h][c], keep = up ? s[k + h][c] : s[k][c];
+                    s[k][c] = keep + __shfl_xor_sync(0xffffffffu, send, h);
+                }
+        }
+#pragma unroll
+        for (int o = B; o < 32; o <<= 1)
+#pragma unroll
+            for (int c = 0; c < C; c++) s[0][c] += __shfl_xor_sync(0xffffffffu, s[0][c], o);
+        if (lane % D / B == bt) {
             for (int q = 0; q < 3; q++) {
-                tu[q] = fmaf(ru[q], b[1][bb], tu[q]);
-                tx[q] = fmaf(rx[q], b[1][bb], tx[q]);
-                ty[q] = fmaf(ru[q], d[1][bb], ty[q]);
+                U[q] = s[0][q];
+                if constexpr (JAC)
+                    for (int k = 0; k < 3; k++) J[q][k] = s[0][3 + 3 * k + q];
             }
         }
-#pragma unroll
-        for (int q = 0; q < 3; q++) {
-            au[q] = fmaf(tu[q], b[2][c], au[q]);
-            ax[q] = fmaf(tx[q], b[2][c], ax[q]);
-            ay[q] = fmaf(ty[q], b[2][c], ay[q]);
-            az[q] = fmaf(tu[q], d[2][c], az[q]);
-        }
     }
-    for (int q = 0; q < 3; q++) {
-        U[q] = au[q];
-        J[q][0] = ax[q]; J[q][1] = ay[q]; J[q][2] = az[q];
-    }
+    __syncwarp();   // the slab is rewritten by the next step
 }
 
 // FP64 interpolant in the reference's order (bit-identical to interp) and its Jacobian
@@ -265,12 +333,19 @@ struct SegArgs {
 };
 
 // K forward steps of one droplet; optional checkpoint at the start and trajectory
+// (FP32: eight droplets per warp, see interp_warp; the lanes past the last droplet repeat it)
 template <typename T, bool JAC>
 __global__ void __launch_bounds__(128) k_adj_segment(SegArgs<T> A)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= A.np) return;
-    const int np = A.np;
+    constexpr bool WARP = std::is_same<T, float>::value;
+    constexpr int D = kWarpDrops;
+    __shared__ float4 slabs[WARP ? D * slab_floats<JAC>() : 1];   // four warps
+    const int np = A.np, lane = threadIdx.x & 31;
+    const int own = WARP ? (blockIdx.x * 4 + threadIdx.x / 32) * D + lane % D : blockIdx.x * blockDim.x + threadIdx.x;
+    if (WARP ? own - lane % D >= np : own >= np) return;
+    const int i = min(own, np - 1);
+    const bool store = own < np && (!WARP || lane < D);
+    float *slab = reinterpret_cast<float *>(slabs) + threadIdx.x / 32 * D * slab_floats<JAC>();
     double x[3];
     T V[3], F1[3], F2[3], U1[3], U2[3], U3[3];
     const T dt = (T)A.dt, g = (T)A.g, tau = (T)A.tau[i];
@@ -287,7 +362,7 @@ __global__ void __launch_bounds__(128) k_adj_segment(SegArgs<T> A)
             U3[c] = A.in.s[(15 + c) * np + i];
         }
     }
-    if (A.ckpt.x && !A.first) {
+    if (A.ckpt.x && !A.first && store) {
         for (int c = 0; c < 3; c++) {
             A.ckpt.x[c * np + i] = x[c];
             A.ckpt.s[(0 + c) * np + i] = V[c];
@@ -305,9 +380,13 @@ __global__ void __launch_bounds__(128) k_adj_segment(SegArgs<T> A)
         T U0[3];
         if constexpr (JAC) {
             T J[3][3];
-            interp_jac(A.F, x, U0, J);
-            for (int q = 0; q < 3; q++)
-                for (int k = 0; k < 3; k++) A.TJ[((int64_t)j * 9 + 3 * q + k) * np + i] = J[q][k];
+            if constexpr (WARP) interp_warp<true>(A.F, x, U0, J, slab);
+            else interp_jac(A.F, x, U0, J);
+            if (store)
+                for (int q = 0; q < 3; q++)
+                    for (int k = 0; k < 3; k++) A.TJ[((int64_t)j * 9 + 3 * q + k) * np + i] = J[q][k];
+        } else if constexpr (WARP) {
+            interp_warp<false>(A.F, x, U0, nullptr, slab);
         } else {
             interp(A.F, x, U0);
         }
@@ -318,7 +397,7 @@ __global__ void __launch_bounds__(128) k_adj_segment(SegArgs<T> A)
                 U1[c] = U0[c]; U2[c] = U0[c]; U3[c] = U0[c];
             }
         }
-        if (A.TX) {
+        if (A.TX && store) {
             if (j == 0)   // histories before the segment (pre-slots)
                 for (int c = 0; c < 3; c++) {
                     A.TV[2 * slot + c * np + i] = F1[c];
@@ -347,12 +426,12 @@ __global__ void __launch_bounds__(128) k_adj_segment(SegArgs<T> A)
             U3[c] = U2[c]; U2[c] = U1[c]; U1[c] = U0[c];
         }
     }
-    if (A.TX)
+    if (A.TX && store)
         for (int c = 0; c < 3; c++) {
             A.TX[(A.nstep + 3) * slot + c * np + i] = x[c];
             A.TV[(A.nstep + 3) * slot + c * np + i] = V[c];
         }
-    if (A.out.x)
+    if (A.out.x && store)
         for (int c = 0; c < 3; c++) {
             A.out.x[c * np + i] = x[c];
             A.out.s[(0 + c) * np + i] = V[c];
@@ -963,10 +1042,9 @@ int run_segment(dl_adj *a, int seg, bool record)
         A.TX = nullptr;
         A.TV = A.TU = A.TJ = nullptr;
     }
-    if (record)
-        k_adj_segment<T, true><<<dl_blocks(np, 128), 128, 0, a->stream>>>(A);
-    else
-        k_adj_segment<T, false><<<dl_blocks(np, 128), 128, 0, a->stream>>>(A);
+    const int blk = a->mixed ? dl_blocks(np, 4 * kWarpDrops) : dl_blocks(np, 128);
+    if (record) k_adj_segment<T, true><<<blk, 128, 0, a->stream>>>(A);
+    else k_adj_segment<T, false><<<blk, 128, 0, a->stream>>>(A);
     ACUDA(a, cudaGetLastError());
     return 0;
 }

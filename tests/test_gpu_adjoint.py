@@ -156,3 +156,25 @@ def test_internal_order_is_invisible(n, np_):
         a.close()
     for r in res[1:]:
         assert all(np.array_equal(p_, q) for p_, q in zip(res[0], r))
+
+
+@pytest.mark.parametrize("np_", [1, 7, 9, 33])
+def test_mixed_gather_at_partial_warps(np_):
+    """FP32 gathers eight droplets per warp: counts around a multiple of eight, against FP64.
+    One step's interpolant and Jacobian are sums of 216 FP32 terms, a few 1e-7 of the
+    field; 2e-5 covers the 10 steps and the division by the small displacement."""
+    rng = np.random.default_rng(np_)
+    n = 12
+    u = rng.standard_normal((3, n, n, n))
+    x0, tau = rng.uniform(-3.0, 9.0, (np_, 3)), rng.uniform(0.5, 2.0, np_)
+    out = {}
+    for prec in ("fp64", "mixed"):
+        a = DropletAdjoint(AdjointParams(n=n, nsteps=10, dt=0.01, gravity=1.0, precision=prec, checkpoint_every=4,
+                                         pair_factor=0.0), np_)
+        a.set_field(u)
+        a.set_droplets(x0, tau, np.full(np_, 1e-6))
+        loss, _ = a.forward()
+        out[prec] = (np.array([loss]), *a.final_state(), *a.backward())
+        a.close()
+    for p, q in zip(out["mixed"], out["fp64"]):
+        assert rel(p, q) < 2e-5
