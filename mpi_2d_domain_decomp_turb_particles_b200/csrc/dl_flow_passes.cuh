@@ -391,30 +391,41 @@ __global__ void __launch_bounds__(128) k_low(ZArgs A)
     }
     if (!row || ky * ky + kz * kz > sphere_lim(A.nek)) return;
     const int64_t sc = (int64_t)n * n * A.px, m = (int64_t)i * A.px;
-    if (A.det && box)
-        for (int x = 1; x <= 2; x++) {
-            const int sh = ik2_of((double)(x * x + ky * ky + kz * kz));
-            if (sh > 2) continue;
-            const double f = sh == 1 ? scale[1] : scale[2];
-            for (int c = 0; c < 3; c++) {
-                double2 v = A.u[c * sc + m + x];
-                A.u[c * sc + m + x] = make_double2(v.x * f, v.y * f);
-            }
-        }
-    // the thread of the lower index of each conjugate pair averages both
+    // the thread of the lower index of each conjugate pair averages both; all loads first
     const int64_t mp = ((int64_t)((n - y) % n) * n + (n - z) % n) * A.px;
-    if (mp < m) return;
-    const int sh = box ? ik2_of((double)(ky * ky + kz * kz)) : 0;
-    const double f = A.det && sh == 1 ? scale[1] : (A.det && sh == 2 ? scale[2] : 1.0);
+    const int k2 = ky * ky + kz * kz;
+    const bool scaled = A.det && box, pair = mp >= m;
+    double2 v[3][3], b[3];
+#pragma unroll
     for (int c = 0; c < 3; c++) {
-        double2 a = A.u[c * sc + m], b = A.u[c * sc + mp];
-        if (f != 1.0) {
-            a = make_double2(a.x * f, a.y * f);
-            b = make_double2(b.x * f, b.y * f);
+        if (pair) {
+            v[c][0] = A.u[c * sc + m];
+            b[c] = A.u[c * sc + mp];
         }
-        double2 v = make_double2(0.5 * (a.x + b.x), 0.5 * (a.y - b.y));
-        if (i == 0) v = make_double2(0.0, 0.0);
-        A.u[c * sc + m] = v;
-        A.u[c * sc + mp] = make_double2(v.x, -v.y);
+        if (scaled) {
+            v[c][1] = A.u[c * sc + m + 1];
+            v[c][2] = A.u[c * sc + m + 2];
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+        if (scaled)
+            for (int x = 1; x <= 2; x++) {
+                const int q2 = x * x + k2;   // shells 1, 2: k^2 = 1, 2 and 3..6
+                if (q2 > 6) continue;
+                const double f = q2 <= 2 ? scale[1] : scale[2];
+                A.u[c * sc + m + x] = make_double2(v[c][x].x * f, v[c][x].y * f);
+            }
+        if (!pair) continue;
+        double2 a = v[c][0], p = b[c];
+        if (scaled && k2 >= 1 && k2 <= 6) {
+            const double f = k2 <= 2 ? scale[1] : scale[2];
+            a = make_double2(a.x * f, a.y * f);
+            p = make_double2(p.x * f, p.y * f);
+        }
+        a = make_double2(0.5 * (a.x + p.x), 0.5 * (a.y - p.y));
+        if (i == 0) a = make_double2(0.0, 0.0);
+        A.u[c * sc + m] = a;
+        A.u[c * sc + mp] = make_double2(a.x, -a.y);
     }
 }
