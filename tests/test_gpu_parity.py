@@ -341,3 +341,27 @@ def test_coalescence_growth_mode_matches_oracle():
     assert merged > 0
     # COALESCE conserves droplet mass: a^3 = a1^3 + a2^3 (partlib.f90:3684)
     assert abs(np.sum(g.get_particles()["yp"][:, 6] ** 3) - mass0) <= 1e-12 * mass0
+
+
+@pytest.mark.parametrize("n,pad", [(13, 2), (32, 0), (37, 5), (70, 2), (130, 1), (260, 2)])
+def test_field_conversion_at_ragged_sizes(n, pad):
+    """The padded copy of a field (rows shorter and longer than a block's threads, odd row
+    pitches, periodic images in x, y and z): INTERPOLATE equals the oracle bit for bit for
+    droplets all over the box and at its faces."""
+    p = dense_params(n=n, npart=400)
+    g, o = Partlib(p), orc.Oracle(**p.oracle_kwargs())
+    g.part_init()
+    o.part_init()
+    rng = np.random.default_rng(n)
+    yp = g.get_particles()["yp"]
+    yp[:200, :3] = rng.choice([0.0, 1e-9, 2 * np.pi - 1e-9], (200, 3))
+    g.set_particles(yp)
+    o.yp[:400] = yp
+    g.prepare_interp()
+    o.prepare_interp()
+    for k in range(3):
+        v = rng.standard_normal((n, n, n + pad))
+        g.interpolate(v, k + 1)
+        o.interpolate(v, k + 1)
+    assert np.array_equal(g.get_particles()["vp"], o.vp[:400])
+    g.close()
