@@ -390,8 +390,8 @@ constexpr int COLL_SBUF = 1024;   // block buffer of the search pass (candidates
 // the trajectory tests with the reference's arithmetic; every output slot is taken by an
 // atomic and the detection order is restored afterwards by the loop key, as before.  An
 // owner goes on the removal list once (flag per droplet), after its first collision.
-template <typename T>
-__device__ __forceinline__ unsigned coll_search(const CollArgs<T> &A, int sa, int4 *sbuf, int *sn)
+template <typename T, int P>
+__device__ __forceinline__ unsigned coll_search(const CollArgs<T> &A, int sa, int part, int4 *sbuf, int *sn)
 {
     const int4 ida = A.pk_id[sa];
     if (ida.w != 0) return 0u;   // a ghost owns no search
@@ -417,58 +417,57 @@ __device__ __forceinline__ unsigned coll_search(const CollArgs<T> &A, int sa, in
         }
     };
 
-    for (int jj = -A.jmax; jj <= A.jmax; jj++) {
+    for (int r = part; r < nj * nk; r += P) {   // this thread's share of the rows of cells
+        const int jj = r / nk - A.jmax, kk = r % nk - A.kmax;
         const int iy2 = iy + jj;
         if (iy2 < 1 - D.ny_coll || iy2 > D.ncd + D.ny_coll) continue;
-        for (int kk = -A.kmax; kk <= A.kmax; kk++) {
-            const int iz2 = iz + kk;
-            if (iz2 < 1 - D.nz_coll || iz2 > D.ncd + D.nz_coll) continue;
-            if (iz2 < 1) continue;
-            if (iz2 <= D.ncd && iy2 < 1) continue;
-            const int row = row_of(D, iy2, iz2);
-            // up to three x ranges: [lo, hi] inside the box and the wrapped parts, with shift sx
-            const int lo_raw = ix - A.imax, hi_raw = ix + A.imax;
+        const int iz2 = iz + kk;
+        if (iz2 < 1 - D.nz_coll || iz2 > D.ncd + D.nz_coll) continue;
+        if (iz2 < 1) continue;
+        if (iz2 <= D.ncd && iy2 < 1) continue;
+        const int row = row_of(D, iy2, iz2);
+        // up to three x ranges: [lo, hi] inside the box and the wrapped parts, with shift sx
+        const int lo_raw = ix - A.imax, hi_raw = ix + A.imax;
 #pragma unroll 1
-            for (int q = 0; q < 3; q++) {
-                int lo, hi, isx;
-                if (q == 0) {
-                    lo = max(1, lo_raw); hi = min(D.ncd, hi_raw); isx = 0;
-                } else if (q == 1) {
-                    if (lo_raw >= 1) continue;
-                    lo = lo_raw + D.ncd; hi = D.ncd; isx = -1;
-                } else {
-                    if (hi_raw <= D.ncd) continue;
-                    lo = 1; hi = hi_raw - D.ncd; isx = 1;
+        for (int q = 0; q < 3; q++) {
+            int lo, hi, isx;
+            if (q == 0) {
+                lo = max(1, lo_raw); hi = min(D.ncd, hi_raw); isx = 0;
+            } else if (q == 1) {
+                if (lo_raw >= 1) continue;
+                lo = lo_raw + D.ncd; hi = D.ncd; isx = -1;
+            } else {
+                if (hi_raw <= D.ncd) continue;
+                lo = 1; hi = hi_raw - D.ncd; isx = 1;
+            }
+            const double sx = (double)isx;
+            int s0, s1;
+            cell_range(A.cell_start, D, row, lo, hi, s0, s1);
+            for (int s = s0; s < s1; s++) {
+                const int4 idb = A.pk_id[s];
+                const int ix2 = idb.z;
+                if (ix2 < lo) continue;
+                if (ix2 > hi) break;
+                if (idb.w == 0 && idb.y <= refa) continue;   // ih2 <= ih1
+                const int ii = isx == 0 ? ix2 - ix : (isx < 0 ? ix2 - D.ncd - ix : ix2 + D.ncd - ix);
+                ncand++;
+                const double4 pb = A.pk_x[s];
+                double xd[3];
+                xd[0] = xa[0] - (pb.x + sx * D.hx);
+                xd[1] = xa[1] - pb.y;
+                xd[2] = xa[2] - pb.z;
+                const double dnij0 = sqrt(xd[0] * xd[0] + xd[1] * xd[1] + xd[2] * xd[2]);
+                const double rcoll = ra + pb.w;
+                bool keep = dnij0 <= 10 * rcoll;
+                if (!keep && abs(ii) <= 1 && abs(jj) <= 1 && abs(kk) <= 1) {
+                    const int src = idb.x;
+                    const double dmb[3] = {(double)A.dm[0][src], (double)A.dm[1][src], (double)A.dm[2][src]};
+                    const double dmove_b = sqrt(dmb[0] * dmb[0] + dmb[1] * dmb[1] + dmb[2] * dmb[2]);
+                    keep = dnij0 <= rcoll + dmove_a + dmove_b;
                 }
-                const double sx = (double)isx;
-                int s0, s1;
-                cell_range(A.cell_start, D, row, lo, hi, s0, s1);
-                for (int s = s0; s < s1; s++) {
-                    const int4 idb = A.pk_id[s];
-                    const int ix2 = idb.z;
-                    if (ix2 < lo) continue;
-                    if (ix2 > hi) break;
-                    if (idb.w == 0 && idb.y <= refa) continue;   // ih2 <= ih1
-                    const int ii = isx == 0 ? ix2 - ix : (isx < 0 ? ix2 - D.ncd - ix : ix2 + D.ncd - ix);
-                    ncand++;
-                    const double4 pb = A.pk_x[s];
-                    double xd[3];
-                    xd[0] = xa[0] - (pb.x + sx * D.hx);
-                    xd[1] = xa[1] - pb.y;
-                    xd[2] = xa[2] - pb.z;
-                    const double dnij0 = sqrt(xd[0] * xd[0] + xd[1] * xd[1] + xd[2] * xd[2]);
-                    const double rcoll = ra + pb.w;
-                    bool keep = dnij0 <= 10 * rcoll;
-                    if (!keep && abs(ii) <= 1 && abs(jj) <= 1 && abs(kk) <= 1) {
-                        const int src = idb.x;
-                        const double dmb[3] = {(double)A.dm[0][src], (double)A.dm[1][src], (double)A.dm[2][src]};
-                        const double dmove_b = sqrt(dmb[0] * dmb[0] + dmb[1] * dmb[1] + dmb[2] * dmb[2]);
-                        keep = dnij0 <= rcoll + dmove_a + dmove_b;
-                    }
-                    if (keep) {
-                        const int loopkey = ((ii + A.imax) * nj + (jj + A.jmax)) * nk + (kk + A.kmax);
-                        emit(make_int4(sa, s, loopkey, isx));
-                    }
+                if (keep) {
+                    const int loopkey = ((ii + A.imax) * nj + (jj + A.jmax)) * nk + (kk + A.kmax);
+                    emit(make_int4(sa, s, loopkey, isx));
                 }
             }
         }
@@ -641,17 +640,23 @@ __device__ __forceinline__ void coll_pair(const CollArgs<T> &A, int4 r)
     }
 }
 
-// Search pass: one thread per sorted entry (owners in cell order share their neighbour rows
-// in L1); the list goes through a block buffer, one global atomic per block
-template <typename T>
+// Search pass: P threads per sorted entry (owners in cell order share their neighbour rows
+// in L1); the list goes through a block buffer, one global atomic per block.  One thread reads
+// its nine rows of cells one after the other, three dependent loads each; where the
+// droplets do not fill the chip several times over, four threads share the rows
+// (kCollSplit entries).
+// 20,000 droplets in 64^3 24 -> 12 us, 100,000 in 128^3 43 -> 30; at 200,000 both take 62, at
+// 1M one thread takes 200 and four 263
+constexpr int kCollSplit = 150000;
+template <typename T, int P>
 __global__ void __launch_bounds__(128) k_coll_search(CollArgs<T> A)
 {
     __shared__ int4 sbuf[COLL_SBUF];
     __shared__ int sn, sbase;
     if (threadIdx.x == 0) sn = 0;
     __syncthreads();
-    const int sa = blockIdx.x * blockDim.x + threadIdx.x;
-    const unsigned ncand = sa < A.ne ? coll_search(A, sa, sbuf, &sn) : 0u;
+    const int sa = (blockIdx.x * blockDim.x + threadIdx.x) / P;
+    const unsigned ncand = sa < A.ne ? coll_search<T, P>(A, sa, threadIdx.x % P, sbuf, &sn) : 0u;
     const unsigned tot = __reduce_add_sync(0xffffffffu, ncand);
     if ((threadIdx.x & 31) == 0 && tot) atomicAdd(A.cand, (unsigned long long)tot);
     __syncthreads();
@@ -1254,7 +1259,8 @@ static int collision_t(dl_ctx *c, dl_coll_report *rep)
         DL_CUDA(c, cudaMemsetAsync(c->coll_n, 0, 2 * sizeof(int), c->stream));
         if (c->nps > 0) {
             DL_CUDA(c, cudaMemsetAsync(c->coll_flag, 0, sizeof(int) * (size_t)c->nps, c->stream));
-            k_coll_search<T><<<dl_blocks(A.ne, t), t, 0, c->stream>>>(A);
+            if (A.ne <= kCollSplit) k_coll_search<T, 4><<<dl_blocks(4 * (long)A.ne, t), t, 0, c->stream>>>(A);
+            else k_coll_search<T, 1><<<dl_blocks(A.ne, t), t, 0, c->stream>>>(A);
             DL_CHECK_LAUNCH(c);
             k_coll_eval<T><<<4 * c->num_sms, 256, 0, c->stream>>>(A);
             DL_CHECK_LAUNCH(c);

@@ -157,9 +157,14 @@ __global__ void k_nei_scatter(int nnz, const NeiApp *app, const int *start, int 
 // truncation spheres leaves before the square root: the walk spends its time on instructions
 // of candidates that become no entry (312 -> 193 us at 256^3 / 1M, 1.5 -> 1.0 ms at
 // 512^3 / 5M).  9 CTAs per SM: 193 us, against 206 at 10 (spills), 197 at 8 and 209 at 7.
+// P threads share an owner's rows, as in the collision search: over few droplets one thread's
+// chain of rows is what the walk waits for (20,000 droplets in 64^3: 53 -> 21 us with four; both
+// take 19 at 100,000 in 128^3)
+constexpr int kWalkSplit = 150000;
+template <int P>
 __global__ void __launch_bounds__(128, 9) k_nei_walk(NeiArgs A)
 {
-    const int sa = blockIdx.x * blockDim.x + threadIdx.x;
+    const int sa = (blockIdx.x * blockDim.x + threadIdx.x) / P, part = threadIdx.x % P;
     if (sa >= A.ne) return;
     const int4 ida = A.pk_id[sa];
     if (ida.y >= A.nps) return;   // a ghost owns no list
@@ -214,41 +219,52 @@ __global__ void __launch_bounds__(128, 9) k_nei_walk(NeiArgs A)
     const int k0 = max(klo, cell_below(xa[2], reach, cz)), k1 = min(khi, cell_above(xa[2], reach, cz));
     const int mlo = max(1, wlo), mhi = min(D.ncd, whi);   // the part inside 1..ncd
     const double reach2 = reach * reach * (1.0 + 1.0e-12);
-    for (int j = j0; j <= j1; j++) {
-        const double gy = fmax(0.0, fmax((j - 1) * cy - xa[1], xa[1] - j * cy) - 1.0e-6 * cy);
-        for (int k = k0; k <= k1; k++) {
-            // rows whose cells lie beyond the reach in (y, z): the corners of the window
-            const double gz = fmax(0.0, fmax((k - 1) * cz - xa[2], xa[2] - k * cz) - 1.0e-6 * cz);
-            if (gy * gy + gz * gz > reach2) continue;
-            const int row = nei_row(D, j, k);
-            const int jrel = j - (iy - D.ny_max), krel = k - (iz - D.nz_max);
-            if (mlo <= mhi) {
-                int s0, s1;
-                cell_range(A.cell_start, D, row, mlo, mhi, s0, s1);
-                for (int s = s0; s < s1; s++) {
-                    const int ix2 = A.pk_id[s].z;
-                    if (ix2 < mlo) continue;
-                    if (ix2 > mhi) break;
-                    visit(s, 0.0, 0, jrel, krel);
-                }
+    // one row of cells; gy: its distance to the owner in y
+    auto walk_row = [&](int j, int k, double gy) {
+        // rows whose cells lie beyond the reach in (y, z): the corners of the window
+        const double gz = fmax(0.0, fmax((k - 1) * cz - xa[2], xa[2] - k * cz) - 1.0e-6 * cz);
+        if (gy * gy + gz * gz > reach2) return;
+        const int row = nei_row(D, j, k);
+        const int jrel = j - (iy - D.ny_max), krel = k - (iz - D.nz_max);
+        if (mlo <= mhi) {
+            int s0, s1;
+            cell_range(A.cell_start, D, row, mlo, mhi, s0, s1);
+            for (int s = s0; s < s1; s++) {
+                const int ix2 = A.pk_id[s].z;
+                if (ix2 < mlo) continue;
+                if (ix2 > mhi) break;
+                visit(s, 0.0, 0, jrel, krel);
             }
-            // the parts that wrap around x (owners within reach of an x face)
-            if (wlo < 1) {
-                const int lo = wlo + D.ncd;
-                int s0, s1;
-                cell_range(A.cell_start, D, row, lo, D.ncd, s0, s1);
-                for (int s = s0; s < s1; s++)
-                    if (A.pk_id[s].z >= lo) visit(s, -1.0, -D.ncd, jrel, krel);
+        }
+        // the parts that wrap around x (owners within reach of an x face)
+        if (wlo < 1) {
+            const int lo = wlo + D.ncd;
+            int s0, s1;
+            cell_range(A.cell_start, D, row, lo, D.ncd, s0, s1);
+            for (int s = s0; s < s1; s++)
+                if (A.pk_id[s].z >= lo) visit(s, -1.0, -D.ncd, jrel, krel);
+        }
+        if (whi > D.ncd) {
+            const int hi = whi - D.ncd;
+            int s0, s1;
+            cell_range(A.cell_start, D, row, 1, hi, s0, s1);
+            for (int s = s0; s < s1; s++) {
+                if (A.pk_id[s].z > hi) break;
+                visit(s, 1.0, D.ncd, jrel, krel);
             }
-            if (whi > D.ncd) {
-                const int hi = whi - D.ncd;
-                int s0, s1;
-                cell_range(A.cell_start, D, row, 1, hi, s0, s1);
-                for (int s = s0; s < s1; s++) {
-                    if (A.pk_id[s].z > hi) break;
-                    visit(s, 1.0, D.ncd, jrel, krel);
-                }
-            }
+        }
+    };
+    auto gap_y = [&](int j) { return fmax(0.0, fmax((j - 1) * cy - xa[1], xa[1] - j * cy) - 1.0e-6 * cy); };
+    if constexpr (P == 1) {
+        for (int j = j0; j <= j1; j++) {
+            const double gy = gap_y(j);
+            for (int k = k0; k <= k1; k++) walk_row(j, k, gy);
+        }
+    } else if (k0 <= k1) {
+        for (int j = j0, k = k0 + part;; k += P) {   // this thread's share of the rows
+            for (; k > k1; k -= k1 - k0 + 1) j++;
+            if (j > j1) break;
+            walk_row(j, k, gap_y(j));
         }
     }
 }
@@ -1882,7 +1898,8 @@ int launch_nei_list(dl_ctx *c)
         k_rad_max<<<std::min(dl_blocks(nps, 256), 4 * c->num_sms), 256, 0, c->stream>>>(nps, c->rad, d_napp + 1);
         DL_CHECK_LAUNCH(c);
         if (attempt) DL_CUDA(c, cudaMemsetAsync(c->nei_cnt, 0, sizeof(int) * (m + 1), c->stream));
-        k_nei_walk<<<dl_blocks(A.ne, 128), 128, 0, c->stream>>>(A);
+        if (A.ne <= kWalkSplit) k_nei_walk<4><<<dl_blocks(4 * (long)A.ne, 128), 128, 0, c->stream>>>(A);
+        else k_nei_walk<1><<<dl_blocks(A.ne, 128), 128, 0, c->stream>>>(A);
         DL_CHECK_LAUNCH(c);
         // CSR offsets and the largest count (the counts are complete even when the entry
         // buffer overflowed); one read for the entry count and the flags
