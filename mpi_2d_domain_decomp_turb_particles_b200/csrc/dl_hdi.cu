@@ -468,12 +468,21 @@ __global__ void __launch_bounds__(kRedThreads) k_sumsq(int64_t n, const T *x, T 
     finish_reduction(s, partials, out, ticket, sh);
 }
 
+// q = v / h, or v / sqrt(h) when h is a squared norm
 template <typename T>
-__global__ void k_scale_div(int64_t n, const T *v, const T *h, T *q)
+__global__ void k_scale_div(int64_t n, const T *v, const T *h, T *q, int root)
 {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const T inv = (T)1 / *h;
+    const T inv = (T)1 / (root ? (T)sqrt((double)*h) : *h);
     if (i < n) q[i] = v[i] * inv;
+}
+
+// Blocks of a Gram-Schmidt reduction: eight elements per thread, up to kRedGrid blocks.  Each
+// block takes one atomic on the shared ticket, so that a full grid over a short vector is
+// mostly tickets (300,000 elements: 7.8 us with 1184 blocks, 5.4 with 147).
+inline int red_grid(int64_t n)
+{
+    return (int)std::max<int64_t>(1, std::min<int64_t>(kRedGrid, (n + 8 * kRedThreads - 1) / (8 * kRedThreads)));
 }
 
 template <typename T>
@@ -1429,7 +1438,7 @@ template <typename T>
 int sumsq(dl_ctx *c, const T *x, int64_t n, double *out)
 {
     Red<T> R = red_of<T>(c);
-    k_sumsq<T><<<kRedGrid, kRedThreads, 0, c->stream>>>(n, x, R.scalar, R.partials, R.ticket);
+    k_sumsq<T><<<red_grid(n), kRedThreads, 0, c->stream>>>(n, x, R.scalar, R.partials, R.ticket);
     DL_CHECK_LAUNCH(c);
     T v;
     DL_CUDA(c, cudaMemcpyAsync(&v, R.scalar, sizeof(T), cudaMemcpyDeviceToHost, c->stream));
@@ -1508,7 +1517,7 @@ int gmres_iterate(dl_ctx *c, const C *coef, double norm_b, double norm_rhs, doub
     {
         const T nr = (T)norm_rhs;
         DL_CUDA(c, cudaMemcpyAsync(R.scalar, &nr, sizeof(T), cudaMemcpyHostToDevice, c->stream));
-        k_scale_div<T><<<nb, tb, 0, c->stream>>>(n3, Q, R.scalar, Q);
+        k_scale_div<T><<<nb, tb, 0, c->stream>>>(n3, Q, R.scalar, Q, 0);
         DL_CHECK_LAUNCH(c);
     }
     double maxerr = kMaxErr, res = 0.0;
@@ -1523,21 +1532,17 @@ int gmres_iterate(dl_ctx *c, const C *coef, double norm_b, double norm_rhs, doub
             const T *qprev = j > 1 ? Q + (int64_t)(j - 2) * qld : nullptr;
             const T *hprev = j > 1 ? R.h + (j - 2) : nullptr;
             const T *qnext = j <= iter ? Q + (int64_t)(j - 1) * qld : nullptr;
-            k_mgs<T><<<kRedGrid, kRedThreads, 0, c->stream>>>(n3, v, qprev, hprev, qnext, R.h + (j - 1), R.partials,
+            k_mgs<T><<<red_grid(n3), kRedThreads, 0, c->stream>>>(n3, v, qprev, hprev, qnext, R.h + (j - 1), R.partials,
                                                               R.ticket);
             DL_CHECK_LAUNCH(c);
         }
+        // q_{iter+1} = v / H(iter+1, iter), the norm taken on the device
+        k_scale_div<T><<<nb, tb, 0, c->stream>>>(n3, v, R.h + iter, Q + (int64_t)iter * qld, 1);
+        DL_CHECK_LAUNCH(c);
         DL_CUDA(c, cudaMemcpyAsync(hcol.data(), R.h, sizeof(T) * (iter + 1), cudaMemcpyDeviceToHost, c->stream));
         DL_CUDA(c, cudaStreamSynchronize(c->stream));
         for (int j = 1; j <= iter; j++) HH(j, iter) = (double)hcol[j - 1];
         HH(iter + 1, iter) = std::sqrt((double)hcol[iter]);
-        // q_{iter+1} = v / H(iter+1, iter)
-        {
-            const T hn = (T)HH(iter + 1, iter);
-            DL_CUDA(c, cudaMemcpyAsync(R.scalar, &hn, sizeof(T), cudaMemcpyHostToDevice, c->stream));
-            k_scale_div<T><<<nb, tb, 0, c->stream>>>(n3, v, R.scalar, Q + (int64_t)iter * qld);
-            DL_CHECK_LAUNCH(c);
-        }
         // Givens update of the least-squares problem (partlib.f90:2888-2944)
         if (iter == 1) {
             const double nrm = std::sqrt(HH(1, 1) * HH(1, 1) + HH(2, 1) * HH(2, 1));
