@@ -456,21 +456,29 @@ static int allocate_state(dl_ctx *c)
     ALLOC(c->lv_new, sizeof(int) * m);
     ALLOC(c->lv_dev, sizeof(int) * m);
     ALLOC(c->lv_dep, sizeof(int) * m);
-    ALLOC(c->d_err, sizeof(int));
     ALLOC(c->col_work, 2 * sizeof(int));
     c->xfer_cap = std::max<size_t>(3 * (size_t)m + 16, 1 << 20);
     ALLOC(c->xfer64, sizeof(double) * c->xfer_cap);
     ALLOC(c->xfer_i, sizeof(int) * (4 * m + 16));
     // statistics
     c->nbinsz = c->dc.nset * c->dc.nset * DL_NBIN;
-    ALLOC(c->hist_i, sizeof(int) * c->nbinsz);
-    ALLOC(c->hist_d, sizeof(double) * 7 * c->nbinsz);
+    {
+        // one block for what a collision step clears and reads back: candidate total (8 bytes),
+        // list length (2 ints), device error flags and a pad (2 ints), counts, then the histograms
+        const size_t o_hd = (DL_COLL_HEAD + sizeof(int) * (8 + 2 * 100) + 15) / 16 * 16;
+        const size_t o_hi = o_hd + sizeof(double) * 7 * c->nbinsz;
+        ALLOC(c->coll_blk, o_hi + sizeof(int) * c->nbinsz);
+        c->cand = reinterpret_cast<unsigned long long *>(c->coll_blk);
+        c->coll_n = reinterpret_cast<int *>(c->coll_blk + 8);
+        c->d_err = reinterpret_cast<int *>(c->coll_blk + 16);
+        c->counts = reinterpret_cast<int *>(c->coll_blk + DL_COLL_HEAD);
+        c->hist_d = reinterpret_cast<double *>(c->coll_blk + o_hd);
+        c->hist_i = reinterpret_cast<int *>(c->coll_blk + o_hi);
+    }
     ALLOC(c->acc_i, sizeof(int) * c->nbinsz);
     ALLOC(c->acc_d, sizeof(double) * 7 * c->nbinsz);
     ALLOC(c->out_i, sizeof(int) * c->nbinsz);
     ALLOC(c->out_d, sizeof(double) * 7 * c->nbinsz);
-    ALLOC(c->counts, sizeof(int) * (8 + 2 * 100));
-    ALLOC(c->cand, sizeof(unsigned long long));
     c->pair_cap = std::max(c->p.ncollmax, 1024);
     ALLOC(c->pairs, sizeof(PairRec) * c->pair_cap);
     c->contact_cap = c->p.mevent;
@@ -515,15 +523,15 @@ extern "C" int dl_destroy(dl_ctx *c)
     F(c->long_rows); F(c->n_long);
     F(c->brick_start); F(c->brick_cnt); F(c->lhnode); F(c->bg); F(c->ghosts); F(c->d_nghost); F(c->gh_blk); F(c->gh_start); F(c->gh_tag); F(c->pert_tmp); F(c->lv_src); F(c->lv_list); F(c->lv_n);
     F(c->ent_row); F(c->ent_ix); F(c->row_start); F(c->row_fill); F(c->row_ent); F(c->leave_nid);
-    F(c->lv_refs); F(c->lv_old); F(c->lv_new); F(c->lv_dev); F(c->lv_dep); F(c->d_err); F(c->col_work);
-    F(c->xfer64); F(c->xfer_i); F(c->hist_i); F(c->hist_d); F(c->acc_i); F(c->acc_d); F(c->out_i); F(c->out_d);
+    F(c->lv_refs); F(c->lv_old); F(c->lv_new); F(c->lv_dev); F(c->lv_dep); F(c->col_work);
+    F(c->xfer64); F(c->xfer_i); F(c->coll_blk); F(c->acc_i); F(c->acc_d); F(c->out_i); F(c->out_d);
     for (int b = 0; b < 2; b++)
         for (int k = 0; k < 3; k++) F(c->sh_pos[b][k]);
     for (int q = 0; q < 4; q++)
         for (int k = 0; k < 3; k++) { F(c->sh_vel[q][k]); F(c->sh_flu[q][k]); }
     for (int k = 0; k < 3; k++) { F(c->sh_vpv[k]); F(c->sh_dmv[k]); F(c->sh_pert[k]); }
     F(c->sh_rad); F(c->sh_gid); F(c->sh_ref);
-    F(c->counts); F(c->cand); F(c->coll_list); F(c->coll_n); F(c->coll_flag); F(c->pairs); F(c->contacts); F(c->remove_dev); F(c->pair_buf); F(c->pair_ibuf); F(c->mv_acc);
+    F(c->coll_list); F(c->coll_flag); F(c->pairs); F(c->contacts); F(c->remove_dev); F(c->pair_buf); F(c->pair_ibuf); F(c->mv_acc);
     F(c->ovl_list); F(c->ovl_cnt); F(c->fpad_own);
     F(c->nei_cnt); F(c->nei_start); F(c->nei_idx); F(c->nei_coef); F(c->nei_coef64); F(c->overlap_flag);
     F(c->kry); F(c->xg); F(c->rg); F(c->bg64); F(c->tmp64); F(c->wv); F(c->xt); F(c->dots); F(c->arn); F(c->co_buf); F(c->scan_buf); F(c->rmax_dev);

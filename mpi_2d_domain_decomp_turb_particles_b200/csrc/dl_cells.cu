@@ -678,6 +678,22 @@ __global__ void __launch_bounds__(256) k_coll_eval(CollArgs<T> A)
         coll_pair(A, A.clist[k]);
 }
 
+// What a collision step starts from: counters, histograms and removal flags at zero (one
+// launch in place of six memsets; with one read-back in place of four, 25 us of a 64^3 step)
+__global__ void __launch_bounds__(256) k_coll_clear(int nbinsz, int ncount, int nps, unsigned long long *cand, int *cn,
+                                                    int *counts, int *hist_i, double *hist_d, int *flag)
+{
+    const int i0 = blockIdx.x * blockDim.x + threadIdx.x, st = gridDim.x * blockDim.x;
+    if (i0 == 0) {
+        *cand = 0ull;
+        cn[0] = cn[1] = 0;
+    }
+    for (int i = i0; i < ncount; i += st) counts[i] = 0;
+    for (int i = i0; i < nbinsz; i += st) hist_i[i] = 0;
+    for (int i = i0; i < 7 * nbinsz; i += st) hist_d[i] = 0.0;
+    for (int i = i0; i < nps; i += st) flag[i] = 0;
+}
+
 __global__ void k_accumulate(int nbinsz, const int *hi, const double *hd, int *acc_i, double *acc_d)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1226,10 +1242,6 @@ static int collision_t(dl_ctx *c, dl_coll_report *rep)
         }
         return 0;
     };
-    if (!c->coll_n) {
-        int r = dev_alloc((void **)&c->coll_n, 2 * sizeof(int));
-        if (r) return r;
-    }
     const int want = c->coll_cap_first > 0 ? c->coll_cap_first : std::max(1 << 16, 2 * c->nps);
     if (c->coll_cap < want && !(c->coll_cap_first > 0 && c->coll_list)) {
         if (c->coll_list) cudaFree(c->coll_list);
@@ -1252,30 +1264,25 @@ static int collision_t(dl_ctx *c, dl_coll_report *rep)
         A.cn = c->coll_n;
         A.ccap = c->coll_cap;
         A.cflag = c->coll_flag;
-        DL_CUDA(c, cudaMemsetAsync(c->hist_i, 0, sizeof(int) * nbz, c->stream));
-        DL_CUDA(c, cudaMemsetAsync(c->hist_d, 0, sizeof(double) * 7 * nbz, c->stream));
-        DL_CUDA(c, cudaMemsetAsync(c->counts, 0, sizeof(int) * ncount, c->stream));
-        DL_CUDA(c, cudaMemsetAsync(c->cand, 0, sizeof(unsigned long long), c->stream));
-        DL_CUDA(c, cudaMemsetAsync(c->coll_n, 0, 2 * sizeof(int), c->stream));
+        k_coll_clear<<<std::min(4 * c->num_sms, dl_blocks(std::max(c->nps, 7 * nbz), 256)), 256, 0, c->stream>>>(
+            nbz, ncount, c->nps, c->cand, c->coll_n, c->counts, c->hist_i, c->hist_d, c->coll_flag);
+        DL_CHECK_LAUNCH(c);
         if (c->nps > 0) {
-            DL_CUDA(c, cudaMemsetAsync(c->coll_flag, 0, sizeof(int) * (size_t)c->nps, c->stream));
             if (A.ne <= kCollSplit) k_coll_search<T, 4><<<dl_blocks(4 * (long)A.ne, t), t, 0, c->stream>>>(A);
             else k_coll_search<T, 1><<<dl_blocks(A.ne, t), t, 0, c->stream>>>(A);
             DL_CHECK_LAUNCH(c);
             k_coll_eval<T><<<4 * c->num_sms, 256, 0, c->stream>>>(A);
             DL_CHECK_LAUNCH(c);
         }
-        // counts, the list length and the candidate total in one batch of copies into
-        // pinned staging (with everything the host bookkeeping needs)
-        hs = static_cast<char *>(dl_host_stage(c, sizeof(int) * ncount + 16));
+        // counts, the list length, the candidate total and the error flags in one copy into pinned
+        // staging
+        hs = static_cast<char *>(dl_host_stage(c, sizeof(int) * ncount + DL_COLL_HEAD));
         if (!hs) return dl_fail(c, DL_E_ALLOC, "cudaHostAlloc of the staging buffer failed");
-        DL_CUDA(c, cudaMemcpyAsync(hs, c->cand, sizeof(unsigned long long), cudaMemcpyDeviceToHost, c->stream));
-        DL_CUDA(c, cudaMemcpyAsync(hs + 8, c->d_err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-        DL_CUDA(c, cudaMemcpyAsync(hs + 12, c->coll_n, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-        DL_CUDA(c, cudaMemcpyAsync(hs + 16, c->counts, sizeof(int) * ncount, cudaMemcpyDeviceToHost, c->stream));
+        DL_CUDA(c, cudaMemcpyAsync(hs, c->coll_blk, DL_COLL_HEAD + sizeof(int) * ncount, cudaMemcpyDeviceToHost,
+                                   c->stream));
         DL_CUDA(c, cudaStreamSynchronize(c->stream));
         int nlist = 0;
-        memcpy(&nlist, hs + 12, sizeof(int));
+        memcpy(&nlist, hs + 8, sizeof(int));
         if (nlist <= c->coll_cap) break;
         // the list overflowed and nothing was evaluated: enlarge it and search again
         if (attempt >= 2) return dl_fail(c, DL_E_CAPACITY, "COLLISION_DET: candidate list overflow");
@@ -1292,11 +1299,11 @@ static int collision_t(dl_ctx *c, dl_coll_report *rep)
     unsigned long long cand;
     memcpy(&cand, hs, sizeof(cand));
     int derr;
-    memcpy(&derr, hs + 8, sizeof(int));
+    memcpy(&derr, hs + 16, sizeof(int));
     if (derr & DL_DERR_LONG_ROW)   // the cell list this search read was not fully sorted
         return dl_fail(c, DL_E_CAPACITY, "HEADLIST: more than 4096 droplets in one row of cells");
     std::vector<int> cnt(ncount);
-    memcpy(cnt.data(), hs + 16, sizeof(int) * ncount);
+    memcpy(cnt.data(), hs + DL_COLL_HEAD, sizeof(int) * ncount);
     if (cnt[6]) return dl_fail(c, DL_E_CAPACITY, "COLLISION_DET: pair, contact or removal buffer full");
     const int npairs = cnt[3], ncontact = cnt[4], nremove = cnt[5];
     if (npairs > c->p.ncollmax)

@@ -174,6 +174,7 @@ struct dl_ctx {
     double *hist_d;              // 7 sums: per call [7*nbinsz], accumulated, written
     int *acc_i, *out_i;
     double *acc_d, *out_d;
+    char *coll_blk;              // one allocation: cand, coll_n, d_err, counts, hist_d, hist_i
     int *counts;                 // icc[3], colltype[nset^2], nir[nset^2], npairs, ncontact, overflow, ...
     unsigned long long *cand;
     int4 *coll_list;             // candidate pairs of the collision search (sorted entries, loop key, x shift)
@@ -344,6 +345,7 @@ int launch_periodic(dl_ctx *c);
 int launch_set_positions(dl_ctx *c, const std::vector<int> &refs, const std::vector<double> &xyz, int clear_leave);
 int launch_periodic_reorder(dl_ctx *c);
 int dl_check_device_errors(dl_ctx *c);
+#define DL_COLL_HEAD 24          // bytes of coll_blk before counts
 #define DL_DERR_REORDER 1        // PERIODIC bookkeeping mismatch
 #define DL_DERR_TMA_TIMEOUT 2    // an interpolation tile wait ran out (the tiles' droplets were skipped)
 #define DL_DERR_LONG_ROW 4       // a cell-list row longer than the shared-memory sort holds
