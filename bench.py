@@ -694,8 +694,8 @@ def config4_bench(dev, torch, steps=4):
     flow kernels."""
     import numpy as np
     from mpi_2d_domain_decomp_turb_particles_b200 import Partlib, ParticleParams
-    from mpi_2d_domain_decomp_turb_particles_b200.bytes_model import (advance_bytes, flow_cross_bytes,
-                                                                      flow_update_bytes, interp_bytes)
+    from mpi_2d_domain_decomp_turb_particles_b200.bytes_model import (advance_bytes, flow_pass_bytes,
+                                                                      interp_bytes)
     from mpi_2d_domain_decomp_turb_particles_b200.flow import Flow
     from mpi_2d_domain_decomp_turb_particles_b200.synthetic import droplets, spectral_field
     n, npart = C4["n"], C4["npart"]
@@ -754,8 +754,8 @@ def config4_bench(dev, torch, steps=4):
                              "interpolation": ph[7], "interp_to_history": ph[0], "advance": ph[6],
                              "cell_list": ph[1], "collision": ph[2], "hdi": ph[3], "periodic_coalesce": ph[4],
                              "overlap": ph[5]},
-            "kernel_gbs": {"k_update (+forcing, finish)": _gbs(flow_update_bytes(n), fparts["update"]),
-                           "k_cross_emit": _gbs(flow_cross_bytes(n), fparts["cross"]),
+            "kernel_gbs": {"k_update_sphere + k_low + k_zinverse": _gbs(flow_pass_bytes(n)["update"], fparts["update"]),
+                           "k_xpass": _gbs(flow_pass_bytes(n)["x"], fparts["cross"]),
                            "k_interp_col": _gbs(interp_bytes("mixed", n, nps), uims),
                            "k_advance_fused": _gbs(advance_bytes("mixed", n, nps), uams)},
             "update_substep_kernels_ms": {"interp": uims, "advance": uams, "both": ukms},

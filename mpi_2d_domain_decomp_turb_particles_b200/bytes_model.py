@@ -16,6 +16,7 @@ inputs of the next transforms: 21 complex words = 336 B per mode.  The cross-pro
 kernel reads u and omega (6 words) and writes u x omega (3 words) per point, 72 B, plus
 the droplet context's padded copy of u (3 words of the droplet precision).
 """
+import math
 
 PER_DROPLET = {"mixed": 188, "fp64": 324}
 FIELD_WORD = {"mixed": 4, "fp64": 8}
@@ -40,6 +41,17 @@ def flow_update_bytes(n: int) -> int:
 
 def flow_cross_bytes(n: int, emit_precision: str = "mixed") -> int:
     return (72 + 3 * FIELD_WORD[emit_precision]) * n ** 3
+
+
+def flow_pass_bytes(n: int, emit_precision: str = "mixed") -> dict:
+    """The flow step's own passes on a grid 2^a or 3 * 2^a (csrc/dl_flow_passes.cuh): what the
+    x pass and the update kernels move, in bytes.  One spectral component is n^2 n/2 complex
+    numbers; inside the dealiasing circle lie pi r^2 / n^2 of its columns and inside the sphere
+    4 pi r^3 / (3 n^3) of its modes, r = int(n/2 - 3/2) + 1/2."""
+    comp, r = 16 * n * n * (n // 2), int(n / 2 - 1.5) + 0.5
+    circle, sphere = math.pi * r * r / n ** 2, 4.0 * math.pi * r ** 3 / (3.0 * n ** 3)
+    x = 9 * comp + 24 * n ** 3 + 3 * FIELD_WORD[emit_precision] * n ** 3
+    return {"x": int(x), "update": int(comp * (15 * sphere + 3 * sphere + 6 * circle))}
 
 
 def collision_bytes(precision: str, npart: int) -> int:
