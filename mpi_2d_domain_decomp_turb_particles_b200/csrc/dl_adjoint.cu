@@ -29,8 +29,8 @@
 // point's velocity and, in FP32, one vector atomic adds a point's gradient.
 //
 // Precision: DL_FP64 everything in FP64 (same operation order as the FP64 reference
-// adjoint, bit-identical forward); DL_MIXED FP32 velocities, histories, field, weights
-// and grid-gradient atomics, FP64 positions, x_bar and tau_bar.
+// adjoint, bit-identical forward); DL_MIXED FP32 field, weights, stored velocities and
+// histories and grid-gradient atomics, FP64 positions, velocity update, x_bar and tau_bar.
 #include "dl_internal.cuh"
 #include "dl_scan.cuh"
 
@@ -145,11 +145,11 @@ __device__ __forceinline__ void interp(const Field<double> &F, const double *x, 
 // each.  With a droplet per lane every load touches up to 32 cache lines, which bounds it.
 // Every group of lanes carries the state of the same eight droplets (32 droplets per warp,
 // each state once, has a serial chain four times as long: 68 us per step of 200,000 droplets).
-// Per step, before (a droplet per lane) and now: 79 -> 50 us forward at 200,000 droplets in
-// 128^3, 12 -> 7 at 20,000 in 64^3, 8.0 -> 2.6 at 500 in 32^3; with the Jacobian 79 -> 80 us at
-// 200,000 (twelve sums per droplet and FP32 issue make up for the loads), the whole backward
-// pass 18 -> 16 us at 20,000 and 12 -> 7 at 500.  Sharing the stores of the recorded
-// trajectory among the lane groups gave nothing.
+// Per step, before (a droplet per lane) and now: 79 -> 51 us forward at 200,000 droplets in
+// 128^3, 12 -> 7 at 20,000 in 64^3, 8.0 -> 2.9 at 500 in 32^3; the whole backward pass
+// 116 -> 119 us at 200,000 (its twelve sums per droplet make up for the loads), 69 -> 52 at
+// 80,000, 12 -> 7 at 500.  Sharing the stores of the recorded trajectory among the lane groups
+// gave nothing.
 // Rows of lane group r: y node r, z nodes 0..5; then y node 4 + (r & 1), z nodes (r >> 1) + 0, 2, 4.
 constexpr int kWarpDrops = 8;
 // floats of a droplet's slab: 0..2 the corner's x, y and z parts (points), 4..9 bz, 10..15 bx,
@@ -335,7 +335,7 @@ struct SegArgs {
 // K forward steps of one droplet; optional checkpoint at the start and trajectory
 // (FP32: eight droplets per warp, see interp_warp; the lanes past the last droplet repeat it)
 template <typename T, bool JAC>
-__global__ void __launch_bounds__(128) k_adj_segment(SegArgs<T> A)
+__global__ void __launch_bounds__(128, std::is_same<T, float>::value && JAC ? 3 : 0) k_adj_segment(SegArgs<T> A)
 {
     constexpr bool WARP = std::is_same<T, float>::value;
     constexpr int D = kWarpDrops;
@@ -346,9 +346,14 @@ __global__ void __launch_bounds__(128) k_adj_segment(SegArgs<T> A)
     const int i = min(own, np - 1);
     const bool store = own < np && (!WARP || lane < D);
     float *slab = reinterpret_cast<float *>(slabs) + threadIdx.x / 32 * D * slab_floats<JAC>();
+    // FP32: the droplet velocity and its update in FP64 within the segment (the checkpoints and
+    // the trajectory hold FP32), so that 100 steps do not add up 100 roundings of the velocity:
+    // the loss takes differences of close droplets' velocities.  Against FP64 after 100 steps:
+    // velocities 1.2e-6 -> 8e-8, gradients with a close pair 8e-5 -> 4e-6; 3 % of the time
     double x[3];
-    T V[3], F1[3], F2[3], U1[3], U2[3], U3[3];
-    const T dt = (T)A.dt, g = (T)A.g, tau = (T)A.tau[i];
+    double V[3], F1[3], F2[3];
+    T U1[3], U2[3], U3[3];
+    const double dt = A.dt, g = A.g, tau = A.tau[i];
     if (A.first) {
         for (int c = 0; c < 3; c++) x[c] = A.x0[3 * i + c];
     } else {
@@ -365,16 +370,17 @@ __global__ void __launch_bounds__(128) k_adj_segment(SegArgs<T> A)
     if (A.ckpt.x && !A.first && store) {
         for (int c = 0; c < 3; c++) {
             A.ckpt.x[c * np + i] = x[c];
-            A.ckpt.s[(0 + c) * np + i] = V[c];
-            A.ckpt.s[(3 + c) * np + i] = F1[c];
-            A.ckpt.s[(6 + c) * np + i] = F2[c];
+            A.ckpt.s[(0 + c) * np + i] = (T)V[c];
+            A.ckpt.s[(3 + c) * np + i] = (T)F1[c];
+            A.ckpt.s[(6 + c) * np + i] = (T)F2[c];
             A.ckpt.s[(9 + c) * np + i] = U1[c];
             A.ckpt.s[(12 + c) * np + i] = U2[c];
             A.ckpt.s[(15 + c) * np + i] = U3[c];
         }
     }
-    const T dtau = dt / ((T)24 * tau);
-    const T dtc = dt / (T)24;
+    const double dtau = dt / (24.0 * tau);
+    const double dtc = dt / 24.0;
+    const double den = 1.0 + 9.0 * dtau, inv = 1.0 / den;
     const int64_t slot = 3 * (int64_t)np;
     for (int j = 0; j < A.nstep; j++) {
         T U0[3];
@@ -392,7 +398,7 @@ __global__ void __launch_bounds__(128) k_adj_segment(SegArgs<T> A)
         }
         if (A.first && j == 0) {   // PART_HISTORY_FVP / FDP first step: every level
             for (int c = 0; c < 3; c++) {
-                V[c] = A.init_velocity ? U0[c] : (c == 0 ? g * tau : (T)0);
+                V[c] = A.init_velocity ? (double)U0[c] : (c == 0 ? g * tau : 0.0);
                 F1[c] = V[c]; F2[c] = V[c];
                 U1[c] = U0[c]; U2[c] = U0[c]; U3[c] = U0[c];
             }
@@ -400,28 +406,29 @@ __global__ void __launch_bounds__(128) k_adj_segment(SegArgs<T> A)
         if (A.TX && store) {
             if (j == 0)   // histories before the segment (pre-slots)
                 for (int c = 0; c < 3; c++) {
-                    A.TV[2 * slot + c * np + i] = F1[c];
-                    A.TV[1 * slot + c * np + i] = F2[c];
+                    A.TV[2 * slot + c * np + i] = (T)F1[c];
+                    A.TV[1 * slot + c * np + i] = (T)F2[c];
                     A.TU[2 * slot + c * np + i] = U1[c];
                     A.TU[1 * slot + c * np + i] = U2[c];
                     A.TU[0 * slot + c * np + i] = U3[c];
                 }
             for (int c = 0; c < 3; c++) {
                 A.TX[(j + 3) * slot + c * np + i] = x[c];
-                A.TV[(j + 3) * slot + c * np + i] = V[c];
+                A.TV[(j + 3) * slot + c * np + i] = (T)V[c];
                 A.TU[(j + 3) * slot + c * np + i] = U0[c];
             }
         }
-        T Vn[3];
+        double Vn[3];
         for (int c = 0; c < 3; c++) {
-            const T tempv = (T)19 * V[c] - (T)5 * F1[c] + F2[c];
-            const T tempd = (T)55 * U0[c] - (T)59 * U1[c] + (T)37 * U2[c] - (T)9 * U3[c];
-            const T unit = c == 0 ? (T)1 : (T)0;
-            Vn[c] = (V[c] + dt * unit * g - dtau * tempv + dtau * tempd) / ((T)1 + (T)9 * dtau);
+            const double tempv = 19.0 * V[c] - 5.0 * F1[c] + F2[c];
+            const double tempd = 55.0 * (double)U0[c] - 59.0 * (double)U1[c] + 37.0 * (double)U2[c] - 9.0 * (double)U3[c];
+            const double unit = c == 0 ? 1.0 : 0.0;
+            const double num = V[c] + dt * unit * g - dtau * tempv + dtau * tempd;
+            Vn[c] = WARP ? num * inv : num / den;   // FP64 contexts: the reference's division
         }
         for (int c = 0; c < 3; c++) {
-            const T dm = dtc * ((T)9 * Vn[c] + (T)19 * V[c] - (T)5 * F1[c] + F2[c]);
-            x[c] = x[c] + (double)dm;
+            const double dm = dtc * (9.0 * Vn[c] + 19.0 * V[c] - 5.0 * F1[c] + F2[c]);
+            x[c] = x[c] + dm;
             F2[c] = F1[c]; F1[c] = V[c]; V[c] = Vn[c];
             U3[c] = U2[c]; U2[c] = U1[c]; U1[c] = U0[c];
         }
@@ -429,14 +436,14 @@ __global__ void __launch_bounds__(128) k_adj_segment(SegArgs<T> A)
     if (A.TX && store)
         for (int c = 0; c < 3; c++) {
             A.TX[(A.nstep + 3) * slot + c * np + i] = x[c];
-            A.TV[(A.nstep + 3) * slot + c * np + i] = V[c];
+            A.TV[(A.nstep + 3) * slot + c * np + i] = (T)V[c];
         }
     if (A.out.x && store)
         for (int c = 0; c < 3; c++) {
             A.out.x[c * np + i] = x[c];
-            A.out.s[(0 + c) * np + i] = V[c];
-            A.out.s[(3 + c) * np + i] = F1[c];
-            A.out.s[(6 + c) * np + i] = F2[c];
+            A.out.s[(0 + c) * np + i] = (T)V[c];
+            A.out.s[(3 + c) * np + i] = (T)F1[c];
+            A.out.s[(6 + c) * np + i] = (T)F2[c];
             A.out.s[(9 + c) * np + i] = U1[c];
             A.out.s[(12 + c) * np + i] = U2[c];
             A.out.s[(15 + c) * np + i] = U3[c];
@@ -951,6 +958,7 @@ struct dl_adj {
     int *cell_cnt = nullptr, *cell_start = nullptr, *cell_fill = nullptr, *cell_key = nullptr, *cell_order = nullptr;
     int *scan_tmp = nullptr;
     int *perm = nullptr;          // internal droplet index -> caller's index
+    void *sort_blk = nullptr;     // scratch of the droplet sort: the pointers below
     unsigned long long *sort_key[2] = {nullptr, nullptr};
     int *sort_order = nullptr;    // the other buffer of perm while sorting
     int *sort_cnt = nullptr, *sort_start = nullptr, *sort_scan = nullptr;
@@ -1288,13 +1296,7 @@ extern "C" int dl_adj_create(const dl_adj_params *p, dl_adj **out)
     ADJ_ALLOC(a->pairs, sizeof(int2) * a->pair_cap);
     ADJ_ALLOC(a->pair_refs, sizeof(int2) * a->pair_cap);
     const size_t ncnt = 256 * (size_t)dl_blocks((long)np, kSortBlock);
-    ADJ_ALLOC(a->sort_key[0], 8 * np);
-    ADJ_ALLOC(a->sort_key[1], 8 * np);
-    ADJ_ALLOC(a->sort_order, sizeof(int) * np);
-    ADJ_ALLOC(a->sort_cnt, sizeof(int) * ncnt);
-    ADJ_ALLOC(a->sort_start, sizeof(int) * (ncnt + 1));
-    ADJ_ALLOC(a->sort_scan, sizeof(int) * 2 * (ncnt / 1024 + 4));
-    ADJ_ALLOC(a->rmax, sizeof(double));
+    ADJ_ALLOC(a->sort_blk, 8 * (2 * np + 1) + sizeof(int) * (np + 2 * ncnt + 1 + 2 * (ncnt / 1024 + 4)));
     ADJ_ALLOC(a->d_npairs, sizeof(int));
     ADJ_ALLOC(a->red, sizeof(double) * 544);
 #undef ADJ_ALLOC
@@ -1302,6 +1304,13 @@ extern "C" int dl_adj_create(const dl_adj_params *p, dl_adj **out)
         dl_adj_destroy(a);
         return r;
     }
+    a->sort_key[0] = reinterpret_cast<unsigned long long *>(a->sort_blk);
+    a->sort_key[1] = a->sort_key[0] + np;
+    a->rmax = reinterpret_cast<double *>(a->sort_key[1] + np);
+    a->sort_order = reinterpret_cast<int *>(a->rmax + 1);
+    a->sort_cnt = a->sort_order + np;
+    a->sort_start = a->sort_cnt + ncnt;
+    a->sort_scan = a->sort_start + ncnt + 1;
     // the buffers were zeroed on the legacy stream; the context's stream does not wait for it
     if (cudaDeviceSynchronize() != cudaSuccess) {
         dl_adj_destroy(a);
@@ -1319,7 +1328,7 @@ extern "C" int dl_adj_destroy(dl_adj *a)
     void *ptrs[] = {a->fpad, a->gpad, a->x0, a->tau, a->rad, a->xs, a->ss, a->ckx, a->cks, a->TX, a->TV, a->TU, a->TJ,
                     a->xbar, a->taubar, a->P, a->Q, a->cell_cnt, a->cell_start, a->cell_fill, a->scan_tmp,
                     a->cell_key, a->cell_order, a->pairs, a->d_npairs, a->red, a->perm, a->pair_refs,
-                    a->sort_key[0], a->sort_key[1], a->sort_order, a->sort_cnt, a->sort_start, a->sort_scan, a->rmax};
+                    a->sort_blk};
     for (void *q : ptrs)
         if (q) cudaFree(q);
     for (auto &e : a->ev)
