@@ -1385,7 +1385,11 @@ extern "C" int dl_adj_set_droplets(dl_adj *a, const double *x0, const double *ta
     const int np = a->p.np;
     const double *dx = x0, *dtau = tau, *drad = radius;
     double *tmp = nullptr;
-    if (!on_device) {
+    if (on_device) {
+        // inputs written on the legacy stream (or a blocking one) come first
+        ACUDA(a, cudaEventRecord(a->ev[0], cudaStreamLegacy));
+        ACUDA(a, cudaStreamWaitEvent(a->stream, a->ev[0], 0));
+    } else {
         ACUDA(a, cudaMallocAsync((void **)&tmp, sizeof(double) * 5 * (size_t)np, a->stream));
         const size_t b = sizeof(double) * (size_t)np;
         ACUDA(a, cudaMemcpyAsync(tmp, x0, 3 * b, cudaMemcpyHostToDevice, a->stream));

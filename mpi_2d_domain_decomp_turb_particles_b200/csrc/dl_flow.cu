@@ -704,7 +704,7 @@ __global__ void k_layout(Grid G, double2 *state, double2 *packed, int in)
     else packed[q] = state[m];
 }
 
-// all three components, caller <-> state, one at a time through a buffer where the layouts differ
+// all three components, caller <-> state, through P where the layouts differ
 int copy_state(dl_flow *f, double2 *state, void *caller, bool in, cudaMemcpyKind k)
 {
     const int64_t packed = (int64_t)f->G.n * f->G.n * f->G.nh;
@@ -713,16 +713,13 @@ int copy_state(dl_flow *f, double2 *state, void *caller, bool in, cudaMemcpyKind
         FCUDA(f, in ? cudaMemcpyAsync(state, caller, b, k, f->stream) : cudaMemcpyAsync(caller, state, b, k, f->stream));
         return 0;
     }
-    double2 *tmp = nullptr;
-    FCUDA(f, cudaMallocAsync((void **)&tmp, sizeof(double2) * packed, f->stream));
-    for (int c = 0; c < 3; c++) {
-        double2 *mine = static_cast<double2 *>(caller) + c * packed;
+    for (int c = 0; c < 3; c++) {   // P is free between steps and holds three packed components
+        double2 *mine = static_cast<double2 *>(caller) + c * packed, *tmp = f->planes + c * packed;
         if (in) FCUDA(f, cudaMemcpyAsync(tmp, mine, sizeof(double2) * packed, k, f->stream));
         k_layout<<<blocks(f->G.M, 256), 256, 0, f->stream>>>(f->G, state + c * f->G.M, tmp, in);
         FCUDA(f, cudaGetLastError());
         if (!in) FCUDA(f, cudaMemcpyAsync(mine, tmp, sizeof(double2) * packed, k, f->stream));
     }
-    FCUDA(f, cudaFreeAsync(tmp, f->stream));
     return 0;
 }
 
