@@ -155,8 +155,9 @@ __global__ void k_nei_scatter(int nnz, const NeiApp *app, const int *start, int 
 // droplets (coalescence can grow droplets past the largest initial radius).  Rows of cells
 // whose (y, z) distance to the owner is beyond it are skipped, and a candidate beyond both
 // truncation spheres leaves before the square root: the walk spends its time on instructions
-// of candidates that become no entry (312 -> 193 us at 256^3 / 1M, 1.5 -> 1.0 ms at
-// 512^3 / 5M).  9 CTAs per SM: 193 us, against 206 at 10 (spills), 197 at 8 and 209 at 7.
+// of candidates that become no entry (256^3 / 1M with radii of 10 to 40 um: 312 -> 193 us in
+// perf/cases.py's coupled case, 204 -> 195 in the bench's; 512^3 / 5M lognormal to 60 um: 1.5 ms
+// as before).  9 CTAs per SM: 193 us, against 206 at 10 (spills), 197 at 8 and 209 at 7.
 // P threads share an owner's rows, as in the collision search: over few droplets one thread's
 // chain of rows is what the walk waits for (20,000 droplets in 64^3: 53 -> 21 us with four; both
 // take 19 at 100,000 in 128^3)
