@@ -38,6 +38,8 @@ template <> struct NarrowT<256> { using P = PlanOf<256, 32, 8, 8, 4>; };
 template <int N> using Wide = typename WideT<N>::P;
 template <int N> using Narrow = typename NarrowT<N>::P;
 
+// Below 32 a tile of 8 kx is half a row and everything is launch latency; above 512 a line needs a
+// fourth stage.  Other even sizes would need radices 5, 7, ...
 inline bool supported(int n)
 {
     switch (n) {

@@ -38,7 +38,9 @@ template <int N>
 __host__ __device__ constexpr int64_t w_plane() { return (int64_t)N * (N / 2) + WPAD; }
 
 // ---- y ------------------------------------------------------------------------------------
-// 8 kx (one 128-byte row) x all y of one field and z plane per block
+// 8 kx (one 128-byte row) x all y of one field and z plane per block.  Bound by DRAM: 0.24 ms for
+// six fields at 256^3 (1.44 GB, 6.0 TB/s), 0.12 for three; the library's strided passes ran at 5.9
+// TB/s over the whole spectrum
 template <int N, int SIGN>
 __global__ void __launch_bounds__(8 * dlfft::Wide<N>::T) k_ypass(double2 *__restrict__ W, double2 *__restrict__ planes,
                                                                   int nek, const double2 *__restrict__ tw)
@@ -232,7 +234,8 @@ struct ZArgs {
     const double2 *tw;
 };
 
-// N_0..2 along z, in place: 8 kx x all z of one component and ky per block
+// N_0..2 along z, in place: 8 kx x all z of one component and ky per block.  0.104 ms at 256^3, 0.63 GB
+// at 6.1 TB/s
 template <int N>
 __global__ void __launch_bounds__(8 * dlfft::Wide<N>::T) k_zforward(ZArgs A)
 {
@@ -257,7 +260,8 @@ __global__ void __launch_bounds__(8 * dlfft::Wide<N>::T) k_zforward(ZArgs A)
 
 constexpr int Z_STATE = 0, Z_STRAIN = 1;
 // The state's six fields along z into W: field 3 + c is u^_c, field c its curl (Z_STATE); or
-// the strain e12, e23, e31 (0..2) and e11, e22, e33 (Z_STRAIN, DISSIP)
+// the strain e12, e23, e31 (0..2) and e11, e22, e33 (Z_STRAIN, DISSIP).  Six blocks side by side
+// read the same three components (out of L2); 0.194 ms at 256^3, 0.85 GB at 4.4 TB/s
 template <int N, int MODE>
 __global__ void __launch_bounds__(8 * dlfft::Wide<N>::T) k_zinverse(ZArgs A)
 {
@@ -311,7 +315,8 @@ __global__ void __launch_bounds__(8 * dlfft::Wide<N>::T) k_zinverse(ZArgs A)
 }
 
 // The update inside the sphere (turb.f90:648-676): Crank-Nicolson + AB2, stochastic forcing,
-// projection, N_old <- N.  Outside, the state and N_old are zero and stay so.
+// projection, N_old <- N.  Outside, the state and N_old are zero and stay so.  0.20 ms at 256^3, 1.05 GB at
+// 5.2 TB/s; k_update over the whole spectrum, with the transform inputs written, 0.45 ms
 __global__ void __launch_bounds__(256) k_update_sphere(ZArgs A)
 {
     const int h = A.n / 2;
@@ -361,7 +366,8 @@ __global__ void __launch_bounds__(256) k_update_sphere(ZArgs A)
 
 // What couples modes: shells 1 and 2 rescaled to the energies f1, f2 (supforDET,
 // flowlib.f90:195-229; from the copies in box, since the modes are rescaled in place), zero
-// mean and the conjugate symmetry of kx = 0 (symmetrize, 233-334).  One thread per (ky, kz).
+// mean and the conjugate symmetry of kx = 0 (symmetrize, 233-334).  One thread per (ky, kz); a few
+// round trips to memory (9 us at 256^3, 5 at 64^3; the serial forcing kernel alone took 26)
 __global__ void __launch_bounds__(128) k_low(ZArgs A)
 {
     __shared__ double e[75];
