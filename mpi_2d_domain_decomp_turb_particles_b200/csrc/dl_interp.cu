@@ -1180,13 +1180,14 @@ __global__ void __launch_bounds__(256) k_convert_field(const double *__restrict_
             const int y = y0 + q * blockDim.y;
             if (y < e) a[q] = src[py * wrap_pad(y, n) + x];
         }
-        const int image = x < DL_PAD_HI ? x + n : (x >= n - DL_PAD_LO ? x - n : x);
 #pragma unroll
         for (int q = 0; q < kConvRows; q++) {
             const int y = y0 + q * blockDim.y;
             if (y >= e) continue;
             dst[opy * y + x] = (T)a[q];
-            if (image != x) dst[opy * y + image] = (T)a[q];
+            // its periodic images: one at most, but below n = DL_PAD_LO + DL_PAD_HI on both sides
+            if (x < DL_PAD_HI) dst[opy * y + x + n] = (T)a[q];
+            if (x >= n - DL_PAD_LO) dst[opy * y + x - n] = (T)a[q];
         }
     }
 }
