@@ -1152,42 +1152,46 @@ __global__ void k_update_pos(int nps, const double *px, const double *py, const 
     qz[d] = pz[d] + (double)dz[d];
 }
 
-// FP64 reference-layout field -> halo-padded copy in precision T (periodic images)
-// (grid: x in blocks of blockDim.x, one padded row (y, z) per blockIdx.y, blockIdx.z)
+// grid plane of padded plane p (grids of DL_PAD_LO and more: at most one period away)
 __device__ __forceinline__ int wrap_pad(int p, int n)
 {
     const int g = p - DL_PAD_LO;
     return g < 0 ? g + n : (g >= n ? g - n : g);
 }
 
-// One component of the reference-layout field into the padded copy.  Streaming: each thread
-// has kConvRows rows in flight and writes the periodic x images from the values it holds; with
-// a thread per padded point (and a third of the blocks for the last 8 of 264 columns) it took
-// 110 us per component at 256^3 mixed; 43 us now, 0.21 GB at 4.9 TB/s.
+// One component of the FP64 reference-layout field into the padded copy in precision T.
+// Streaming: each thread has kConvRows rows in flight and writes the periodic x images from the
+// values it holds; with a thread per padded point (and a third of the blocks for the last 8 of
+// 264 columns) it took 110 us per component at 256^3 mixed; 43 us now, 0.21 GB at 4.9 TB/s.
+// NARROW: grids below DL_PAD_LO + DL_PAD_HI, where a column has images on both sides, at n = 3
+// also two periods away; the others have one at most (256^3 takes 45 us in the general form).
 constexpr int kConvRows = 8;
-template <typename T>
+template <typename T, bool NARROW>
 __global__ void __launch_bounds__(256) k_convert_field(const double *__restrict__ v, int64_t py, int64_t pz, int n,
                                                        T *__restrict__ out, int64_t opy, int64_t opz)
 {
     const int e = n + DL_PAD_LO + DL_PAD_HI, z = blockIdx.y;
     const int y0 = blockIdx.x * (blockDim.y * kConvRows) + threadIdx.y;
-    const double *src = v + pz * wrap_pad(z, n);
+    const auto plane = [n](int p) { return NARROW ? wrapi(p - DL_PAD_LO, n) : wrap_pad(p, n); };
+    const double *src = v + pz * plane(z);
     T *dst = out + opz * z + DL_PAD_LO;
     for (int x = threadIdx.x; x < n; x += blockDim.x) {
         double a[kConvRows];
 #pragma unroll
         for (int q = 0; q < kConvRows; q++) {
             const int y = y0 + q * blockDim.y;
-            if (y < e) a[q] = src[py * wrap_pad(y, n) + x];
+            if (y < e) a[q] = src[py * plane(y) + x];
         }
+        const int image = x < DL_PAD_HI ? x + n : (x >= n - DL_PAD_LO ? x - n : x);
 #pragma unroll
         for (int q = 0; q < kConvRows; q++) {
             const int y = y0 + q * blockDim.y;
             if (y >= e) continue;
             dst[opy * y + x] = (T)a[q];
-            // its periodic images: one at most, but below n = DL_PAD_LO + DL_PAD_HI on both sides
-            if (x < DL_PAD_HI) dst[opy * y + x + n] = (T)a[q];
-            if (x >= n - DL_PAD_LO) dst[opy * y + x - n] = (T)a[q];
+            if (!NARROW && image != x) dst[opy * y + image] = (T)a[q];
+            if (NARROW)
+                for (int i = x - 2 * n; i <= x + 2 * n; i += n)
+                    if (i >= -DL_PAD_LO && i < n + DL_PAD_HI) dst[opy * y + i] = (T)a[q];
         }
     }
 }
@@ -1727,14 +1731,13 @@ int launch_convert_field(dl_ctx *c, int icpt)
     const dim3 block((unsigned)tx, (unsigned)(256 / tx));
     const dim3 grid((unsigned)((e + 256 / tx * kConvRows - 1) / (256 / tx * kConvRows)), (unsigned)e);
     const int k = icpt - 1;
-    if (c->mixed)
-        k_convert_field<float><<<grid, block, 0, c->stream>>>(c->f64[k], c->fpy[k], c->fpz[k], n,
-                                                             (float *)c->fpad + (int64_t)k * c->fp_comp,
-                                                             c->fp_pitch, c->fp_plane);
-    else
-        k_convert_field<double><<<grid, block, 0, c->stream>>>(c->f64[k], c->fpy[k], c->fpz[k], n,
-                                                              (double *)c->fpad + (int64_t)k * c->fp_comp,
-                                                              c->fp_pitch, c->fp_plane);
+    const auto convert = [&](auto *fpad, auto kernel) {
+        kernel<<<grid, block, 0, c->stream>>>(c->f64[k], c->fpy[k], c->fpz[k], n, fpad + (int64_t)k * c->fp_comp,
+                                              c->fp_pitch, c->fp_plane);
+    };
+    const bool narrow = n < DL_PAD_LO + DL_PAD_HI;
+    if (c->mixed) convert((float *)c->fpad, narrow ? k_convert_field<float, true> : k_convert_field<float, false>);
+    else convert((double *)c->fpad, narrow ? k_convert_field<double, true> : k_convert_field<double, false>);
     DL_CHECK_LAUNCH(c);
     return 0;
 }

@@ -368,10 +368,10 @@ def test_field_conversion_at_ragged_sizes(n, pad):
 
 
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
-@pytest.mark.parametrize("n", [4, 5, 6, 7, 8])
+@pytest.mark.parametrize("n", [3, 4, 5, 6, 7, 8])
 def test_field_conversion_on_grids_narrower_than_the_halo(n, precision):
-    """Below n = 8 a column has periodic images on both sides of the padded row.  FP64 bit for
-    bit; mixed within 1e-5 of the largest field value: about 30 FP32 roundings (6e-8) of the
+    """Below n = 8 a column has periodic images on both sides of the padded row, and at n = 3,
+    the smallest grid PART_INIT takes, some planes are two periods away.  FP64 bit for bit; mixed within 1e-5 of the largest field value: about 30 FP32 roundings (6e-8) of the
     field, the three weights and the sums, times the weights' absolute sum, at most 1.4 per
     direction and 2.7 for the three."""
     p = dense_params(n=n, npart=400, precision=precision)
