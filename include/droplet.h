@@ -318,7 +318,10 @@ int dl_flow_get_forcing_state(dl_flow *f, double *b450, int *iseedf, int *iyf, i
 int dl_flow_set_forcing_state(dl_flow *f, const double *b450, int iseedf, int iyf, const int *ivf32);
 /* One time step.  The physical velocity of the state at the start of the step (the field
  * the particle substep of this step interpolates, turb.f90:537-539) is left on the device
- * (dl_flow_velocity) and, when droplets is not NULL, set as that context's field. */
+ * (dl_flow_velocity) and, when droplets is not NULL, set as that context's field.
+ * Every component rounds at its own magnitude, and one that is zero and not driven stays zero.
+ * A flow that does not vary along x or z stays exactly so; along y, on the grids with passes of
+ * their own, to rounding (two neighbouring rows share a transform). */
 int dl_flow_step(dl_flow *f, dl_ctx *droplets);
 /* device pointer to physical component icpt (1..3) of the last step's velocity
  * (n^3, x fastest; pitches n and n*n), NULL before the first step */

@@ -106,12 +106,14 @@ __device__ __forceinline__ void emit_value(F *row, int x, int n, double u)
 }
 
 // Two rows (y, y + 1) of one z plane per group of 3 T threads.  The half spectra A, B of two
-// real lines go through one complex transform of A + i B: thread group p takes components
-// (0, 1) of row p, or component 2 of both rows (p = 2), for the velocity, for the vorticity
-// and for N, 4.5 transforms per row.  The pair has to be of one magnitude, since both round
-// at the larger one's: u beside the vorticity would lose a factor |omega| / |u| (50 at 256^3).
+// real lines go through one complex transform of A + i B: thread group p takes component p of
+// both rows, for the velocity, for the vorticity and for N, 4.5 transforms per row.  Both
+// lines of a pair round at the larger one's magnitude, so they are of one component (the
+// transforms along z and y have rounded its rows alike): beside another component a small one
+// would lose their ratio, and one that is zero would not stay so (and the components (0, 1) of a
+// row took 0.49 ms at 256^3).
 // Bound by the load/store unit and the latency of its phases: 24 16-byte accesses of the SM per
-// element and thread group (0.26 ms at 256^3), 1.6 GB of DRAM (0.25 ms); 0.49 ms, where the
+// element and thread group (0.26 ms at 256^3), 1.6 GB of DRAM (0.25 ms); 0.47 ms, where the
 // library's x transforms and the cross-product kernel took 0.78.
 template <int N, int MODE>
 __global__ void __launch_bounds__(x_threads<N>(), N == 256 ? 2 : 4) k_xpass(XArgs A)
@@ -126,13 +128,11 @@ __global__ void __launch_bounds__(x_threads<N>(), N == 256 ? 2 : 4) k_xpass(XArg
     double2 *reg = sm + unit * 6 * SL;   // lines of the velocity (0..2) and the vorticity (3..5)
     constexpr int64_t fstride = (int64_t)N * N * H;
     double2 *rows = A.P + ((int64_t)z * N + y0) * H;
-    // the pair of lines of this thread group: component and row
-    const int ca = p < 2 ? 0 : 2, cb = p < 2 ? 1 : 2, ra = p < 2 ? p : 0, rb = p < 2 ? p : 1;
     const auto at = [](int i) { return slot_at<P>(i); };
     double2 v[E];
 #pragma unroll 1
     for (int r = 0; r < 2; r++) {
-        const double2 *a = rows + (ca + 3 - 3 * r) * fstride + ra * H, *b = rows + (cb + 3 - 3 * r) * fstride + rb * H;
+        const double2 *a = rows + (p + 3 - 3 * r) * fstride, *b = a + H;
         dlfft::each<P, 0>(t, [&](int i, int m) {
             const int k = dlfft::in_at<P, 0>(t, i, m);
             const int kk = k <= H ? k : N - k;
@@ -150,8 +150,7 @@ __global__ void __launch_bounds__(x_threads<N>(), N == 256 ? 2 : 4) k_xpass(XArg
         sync();
         dlfft::each<P, L>(t, [&](int i, int m) { mine[at(dlfft::out_at<P, L>(t, i, m))] = v[i * RO + m]; });
         if (MODE != X_DISS && r == 0) {
-            double *ua = A.vel + (((int64_t)ca * N + z) * N + y0 + ra) * N;
-            double *ub = A.vel + (((int64_t)cb * N + z) * N + y0 + rb) * N;
+            double *ua = A.vel + (((int64_t)p * N + z) * N + y0) * N, *ub = ua + N;
             dlfft::each<P, L>(t, [&](int i, int m) {
                 const int x = dlfft::out_at<P, L>(t, i, m);
                 ua[x] = v[i * RO + m].x;
@@ -162,10 +161,10 @@ __global__ void __launch_bounds__(x_threads<N>(), N == 256 ? 2 : 4) k_xpass(XArg
                 const int Z[2] = {z + DL_PAD_LO, pad_image(z, N)};
 #pragma unroll 1
                 for (int q = 0; q < 8; q++) {   // both lines and their periodic images in y and z
-                    const int y = y0 + (q & 1 ? rb : ra);
+                    const int y = y0 + (q & 1);
                     const int Yq = q & 2 ? pad_image(y, N) : y + DL_PAD_LO, Zq = q & 4 ? Z[1] : Z[0];
                     if (Yq < 0 || Zq < 0) continue;
-                    F *row = static_cast<F *>(A.fp) + (q & 1 ? cb : ca) * A.fpc + A.fpz * Zq + A.fpy * Yq;
+                    F *row = static_cast<F *>(A.fp) + p * A.fpc + A.fpz * Zq + A.fpy * Yq;
                     dlfft::each<P, L>(t, [&](int i, int m) {
                         emit_value(row, dlfft::out_at<P, L>(t, i, m), N, q & 1 ? v[i * RO + m].y : v[i * RO + m].x);
                     });
@@ -180,11 +179,9 @@ __global__ void __launch_bounds__(x_threads<N>(), N == 256 ? 2 : 4) k_xpass(XArg
         for (int j = p * T + t; j < 2 * N; j += 3 * T) {
             const int r = j / N, x = j - r * N;
             double s[6];
-            for (int h = 0; h < 2; h++) {
-                const double2 a = reg[(3 - 3 * h + r) * SL + at(x)], b = reg[(5 - 3 * h) * SL + at(x)];
-                s[3 * h] = a.x;
-                s[3 * h + 1] = a.y;
-                s[3 * h + 2] = r ? b.y : b.x;
+            for (int c = 0; c < 6; c++) {
+                const double2 a = reg[(c < 3 ? 3 + c : c - 3) * SL + at(x)];
+                s[c] = r ? a.y : a.x;
             }
             double e = 0.0;
             for (int c = 0; c < 6; c++) e = c < 3 ? e + 2.0 * s[c] * s[c] : e + s[c] * s[c];
@@ -193,27 +190,19 @@ __global__ void __launch_bounds__(x_threads<N>(), N == 256 ? 2 : 4) k_xpass(XArg
         return;
     }
     // N = u x omega (turb.f90:634-637)
-    if (p < 2) {
-        dlfft::each<P, 0>(t, [&](int i, int m) {
-            const int x = at(dlfft::in_at<P, 0>(t, i, m));
-            const double2 u = reg[p * SL + x], w = reg[(3 + p) * SL + x], u2 = reg[2 * SL + x], w2 = reg[5 * SL + x];
-            const double uz = p ? u2.y : u2.x, wz = p ? w2.y : w2.x;
-            v[i * RI + m] = make_double2(u.y * wz - uz * w.y, uz * w.x - u.x * wz);
-        });
-    } else {
-        dlfft::each<P, 0>(t, [&](int i, int m) {
-            const int x = at(dlfft::in_at<P, 0>(t, i, m));
-            const double2 u = reg[x], w = reg[3 * SL + x], s = reg[SL + x], q = reg[4 * SL + x];
-            v[i * RI + m] = make_double2(u.x * w.y - u.y * w.x, s.x * q.y - s.y * q.x);
-        });
-    }
+    const double2 *u1 = reg + (p + 1) % 3 * SL, *u2 = reg + (p + 2) % 3 * SL, *w1 = u1 + 3 * SL, *w2 = u2 + 3 * SL;
+    dlfft::each<P, 0>(t, [&](int i, int m) {
+        const int x = at(dlfft::in_at<P, 0>(t, i, m));
+        const double2 a = u1[x], b = u2[x], c = w1[x], d = w2[x];
+        v[i * RI + m] = make_double2(a.x * d.x - b.x * c.x, a.y * d.y - b.y * c.y);
+    });
     __syncthreads();
     double2 *mine = reg + p * SL;
     dlfft::line<P, -1>(t, v, mine, at, A.tw, sync);
     sync();
     dlfft::each<P, L>(t, [&](int i, int m) { mine[at(dlfft::out_at<P, L>(t, i, m))] = v[i * RO + m]; });
     sync();
-    double2 *oa = rows + ca * fstride + ra * H, *ob = rows + cb * fstride + rb * H;
+    double2 *oa = rows + p * fstride, *ob = oa + H;
     for (int k = t; k <= A.nek; k += T) {
         const double2 a = mine[at(k)], b = mine[at(k ? N - k : 0)];
         oa[k] = make_double2(0.5 * (a.x + b.x), 0.5 * (a.y - b.y));

@@ -108,3 +108,63 @@ def test_n_old_outside_the_sphere_is_dropped():
     assert rel(uh, o.uh) < TOL and rel(nold, o.nold) < TOL
     assert not nold[:, o.ik2 > o.nek].any() and not uh[:, o.ik2 > o.nek].any()
     g.close()
+
+
+def spectral_state(n, scale, seed):
+    """Spectra of three real random fields of the given magnitudes, dealiased, on the device."""
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    k, keep = wavenumbers(n)
+    uh = [torch.fft.rfftn(torch.randn((n, n, n), generator=gen, device="cuda", dtype=torch.float64), norm="forward")
+          for _ in range(3)]
+    return torch.stack([torch.where(keep, s * a, 0.0) for s, a in zip(uh, scale)])
+
+
+def wavenumbers(n):
+    k = torch.fft.fftfreq(n, 1.0 / n, device="cuda", dtype=torch.float64)
+    kv = (torch.arange(n // 2 + 1, device="cuda", dtype=torch.float64)[None, None, :], k[None, :, None], k[:, None, None])
+    return kv, torch.floor((kv[0] ** 2 + kv[1] ** 2 + kv[2] ** 2).sqrt() + 0.5) <= int(n / 2 - 1.5)
+
+
+@pytest.mark.parametrize("n,c", [(32, 0), (48, 1), (64, 2), (96, 0), (128, 1), (192, 2), (256, 0), (384, 1)])
+def test_components_keep_their_own_accuracy(n, c):
+    """Component c a million times the others: every component of the velocity and of N is as
+    accurate, against its own norm, as it is where all three are of one magnitude."""
+    kv, keep = wavenumbers(n)
+    g = Flow(n, 1e-3, 1e-4)
+    g.set_spectral(spectral_state(n, [1e6 if q == c else 1.0 for q in range(3)], n).cpu().numpy())
+    uh = torch.from_numpy(g.spectral()[0]).cuda()
+    g.step()
+    nold = torch.from_numpy(g.spectral()[1]).cuda()
+    inv = lambda a: torch.fft.irfftn(a, s=(n,) * 3, norm="forward")   # noqa: E731
+    u = [inv(uh[q]) for q in range(3)]
+    for q, t in enumerate(g.velocity_tensors()):
+        assert float((t - u[q]).norm() / u[q].norm()) < TOL
+    w = [inv(1j * (kv[(q + 1) % 3] * uh[(q + 2) % 3] - kv[(q + 2) % 3] * uh[(q + 1) % 3])) for q in range(3)]
+    for q in range(3):
+        a, b = (q + 1) % 3, (q + 2) % 3
+        ref = torch.where(keep, torch.fft.rfftn(u[a] * w[b] - u[b] * w[a], norm="forward"), 0.0)
+        assert float((nold[q] - ref).norm() / ref.norm()) < TOL
+    g.close()
+
+
+@pytest.mark.parametrize("n", [32, 48, 96, 128, 256])
+@pytest.mark.parametrize("c", [0, 1, 2])
+def test_plane_flow_stays_plane(n, c):
+    """A flow without component c that does not vary along c: exactly so along x and z; along y
+    the two rows of a pair round differently."""
+    kv, keep = wavenumbers(n)
+    a, b = (c + 1) % 3, (c + 2) % 3
+    psi = torch.where(kv[c] == 0, spectral_state(n, (1.0, 1.0, 1.0), c)[0], 0.0)
+    uh = torch.zeros((3, *psi.shape), dtype=torch.complex128, device="cuda")
+    uh[a], uh[b] = 1j * kv[b] * psi, -1j * kv[a] * psi
+    g = Flow(n, 1e-2, 1e-4)
+    g.set_spectral(uh.cpu().numpy())
+    for _ in range(3):
+        g.step()
+    u = g.velocity_tensors()
+    s, nold = (torch.from_numpy(v).cuda() for v in g.spectral())
+    mean = u[a].select(2 - c, 0).unsqueeze(2 - c)
+    parts = [(u[c], u[a]), (u[a] - mean, u[a]), (s[c], s), (nold[c], nold), (torch.where(kv[c] == 0, 0.0, s), s)]
+    for zero, whole in parts:
+        assert float(zero.norm() / whole.norm()) <= (TOL if c == 1 else 0.0)
+    g.close()
