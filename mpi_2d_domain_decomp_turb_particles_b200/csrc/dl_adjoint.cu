@@ -15,7 +15,8 @@
 // Layout and schedule.  One thread per droplet carries its state through a whole
 // segment of K steps in registers (one launch per segment).  The forward pass stores a
 // checkpoint (x, V, V_{-1}, V_{-2}, U_{-1..-3}) at every segment start.  The backward
-// pass walks the segments in reverse: it recomputes the segment from its checkpoint,
+// pass walks the segments in reverse: it recomputes the segment from its checkpoint (the same
+// bits as in the forward pass, in both precisions),
 // storing (x_n, V_n, U_n) and the interpolant's Jacobian dU_n/dx per step (one pass over
 // the stencil gives both), then runs the reverse sweep of the segment with the adjoint
 // state (x_bar, tau_bar and two three-deep shift registers of velocity and
@@ -248,17 +249,22 @@ __device__ __forceinline__ void interp_warp(const Field<float> &F, const double 
             }
         }
         // sums over the warp: the first steps halve the droplets a lane still holds, so that
-        // lane l ends with droplet l % B
+        // lane l ends with droplet l % B.  Lane distances 2, 1, 4, 8, 16 with either B: the
+        // recomputation with the Jacobian then gives the forward pass's velocities bit for bit
 #pragma unroll
-        for (int h = B / 2; h > 0; h >>= 1) {
+        for (int q = 0, done = 0; q < (B == 8 ? 3 : 2); q++) {
+            const int h = q < 2 ? 2 >> q : 4;
             const bool up = lane & h;
 #pragma unroll
-            for (int k = 0; k < h; k++)
+            for (int k = 0; k < B; k++) {
+                if (k & (done | h)) continue;
 #pragma unroll
                 for (int c = 0; c < C; c++) {
                     const float send = up ? s[k][c] : s[k + h][c], keep = up ? s[k + h][c] : s[k][c];
                     s[k][c] = keep + __shfl_xor_sync(0xffffffffu, send, h);
                 }
+            }
+            done |= h;
         }
 #pragma unroll
         for (int o = B; o < 32; o <<= 1)

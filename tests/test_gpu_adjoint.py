@@ -178,3 +178,33 @@ def test_mixed_gather_at_partial_warps(np_):
         a.close()
     for p, q in zip(out["mixed"], out["fp64"]):
         assert rel(p, q) < 2e-5
+
+
+@pytest.mark.parametrize("np_", [1, 8, 33])
+def test_recomputation_repeats_the_forward_pass(np_):
+    """Mixed: the reverse sweep runs along the trajectory that the forward pass took, bit for
+    bit.  All droplets sit half-way between two x planes whose six neighbours' weighted values
+    cancel, so the velocity they see is rounding alone (1e-7 of the field) and another order
+    of the sum gives another velocity.  One step from rest without gravity gives V = 24 d U /
+    (1 + 9 d), d = dt / 24 tau, and a displacement s = 9 dt V / 24; the gradient of the mean
+    of s^2 by tau is then -2 s^2 / (np tau (1 + 9 d)) with the s of the forward pass, if both
+    passes had the same U.  About 20 FP32 roundings lie between: 1e-5."""
+    n, m, dt = 16, 5, 0.1
+    rng = np.random.default_rng(np_)
+    w = np.array([3.0, -25.0, 150.0, 150.0, -25.0, 3.0]) / 256.0   # 6-point weights at 1/2
+    line = np.zeros(n)
+    line[m - 2:m + 4] = rng.uniform(0.5, 1.5, 6)
+    line[m + 3] = -(w[:5] @ line[m - 2:m + 3]) / w[5]
+    u = 1e4 * rng.uniform(0.5, 1.5, (3, n, n, 1)) * line
+    dx = 2 * np.pi / n
+    x0 = np.stack([np.full(np_, (m + 0.5) * dx), *rng.uniform(0.0, 2 * np.pi, (2, np_))], axis=1)
+    tau = rng.uniform(0.05, 0.2, np_)
+    a = DropletAdjoint(AdjointParams(n=n, nsteps=1, dt=dt, gravity=0.0, precision="mixed", pair_factor=0.0), np_)
+    a.set_field(u)
+    a.set_droplets(x0, tau, np.full(np_, 1e-6))
+    a.forward()
+    s2 = ((a.final_state()[0] - x0) ** 2).sum(axis=1)
+    dtau = a.backward()[1]
+    assert (s2 > 0.0).all()
+    assert np.allclose(dtau, -2.0 * s2 / (np_ * tau * (1.0 + 9.0 * dt / (24.0 * tau))), rtol=1e-5, atol=0.0)
+    a.close()
