@@ -14,12 +14,9 @@ template <int N_, int T_, int A, int B, int C = 1>
 struct PlanOf {
     static constexpr int N = N_, S = C > 1 ? 3 : 2, T = T_, R0 = A, R1 = B, R2 = C;
 };
-// Lengths 2^a and 3 * 2^a, two plans each.  Every stage boundary is a write and a read of the
-// line in shared memory, so Wide takes two stages with up to 16 elements per thread: the y
-// pass, which does nothing but the transform, runs at 5.6-6.0 TB/s with it.  Narrow keeps 8
-// elements per thread in three stages: the x and z passes hold their lines in shared memory
-// between the transforms, which limits the threads per SM by lines rather than registers, and
-// twice the threads per line hide twice the latency (256^3: see the kernels).
+// Lengths 2^a and 3 * 2^a.  Every stage boundary is a write and a read of the line in shared
+// memory, so Wide takes two stages with up to 16 elements per thread, three of 8 beyond 256.  The
+// y and z passes run on it everywhere (the transforms alone at 5.6-6.1 TB/s).
 template <int N> struct WideT;
 template <> struct WideT<32> { using P = PlanOf<32, 4, 8, 4>; };
 template <> struct WideT<48> { using P = PlanOf<48, 8, 8, 6>; };
@@ -30,11 +27,14 @@ template <> struct WideT<192> { using P = PlanOf<192, 16, 12, 16>; };
 template <> struct WideT<256> { using P = PlanOf<256, 16, 16, 16>; };
 template <> struct WideT<384> { using P = PlanOf<384, 64, 8, 8, 6>; };
 template <> struct WideT<512> { using P = PlanOf<512, 64, 8, 8, 8>; };
+// Narrow, for the x pass, is Wide but at 128 and 192, where it takes three stages of 8 elements
+// and twice the threads per line: the x pass holds six lines per pair of rows in shared memory,
+// which limits the threads per SM by lines rather than registers.  Flow step with the droplet
+// field, this and Wide: 128^3 203 and 225 us, 192^3 602 and 615.  At 96 the same form takes 101.5
+// and Wide 99.4; at 256 the steps are equal, and DISSIP takes 976 and 946.
 template <int N> struct NarrowT : WideT<N> {};
-template <> struct NarrowT<96> { using P = PlanOf<96, 16, 8, 4, 3>; };
 template <> struct NarrowT<128> { using P = PlanOf<128, 16, 8, 4, 4>; };
 template <> struct NarrowT<192> { using P = PlanOf<192, 32, 8, 8, 3>; };
-template <> struct NarrowT<256> { using P = PlanOf<256, 32, 8, 8, 4>; };
 template <int N> using Wide = typename WideT<N>::P;
 template <int N> using Narrow = typename NarrowT<N>::P;
 
@@ -133,10 +133,6 @@ __device__ __forceinline__ double2 rot48(double2 a)
 
 template <int SIGN, int R>
 struct Dft;
-template <int SIGN>
-struct Dft<SIGN, 1> {
-    static __device__ __forceinline__ void run(double2 *) {}
-};
 template <int SIGN>
 struct Dft<SIGN, 2> {
     static __device__ __forceinline__ void run(double2 *v)

@@ -412,7 +412,7 @@ struct dl_flow {
     int fast = 0;
     double2 *planes = nullptr;   // P
     double2 *box = nullptr;      // modes of the deterministic forcing
-    double2 *tw = nullptr, *tw_wide = nullptr;   // twiddles of the Narrow plan (x) and the Wide one (y, z)
+    double2 *tw = nullptr, *tw_wide = nullptr;   // twiddles of the x plan and the y and z one
     int nold_dirty = 0;          // N_old may hold modes outside the sphere
     double *afor = nullptr;      // device copy of the stochastic forcing amplitudes
     double *spec_part = nullptr;

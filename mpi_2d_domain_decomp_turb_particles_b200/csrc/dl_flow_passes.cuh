@@ -72,11 +72,7 @@ __global__ void __launch_bounds__(8 * dlfft::Wide<N>::T) k_ypass(double2 *__rest
 }
 
 // ---- x ------------------------------------------------------------------------------------
-// Narrow, but for 256: 0.49 ms at two blocks per SM with Wide, 0.57 ms at four with Narrow; at
-// 128, 192, 384 and 512 the two differ by less than the runs do
-template <int N> struct XP { using P = dlfft::Narrow<N>; };
-template <> struct XP<256> { using P = dlfft::Wide<256>; };
-template <int N> using XPlan = typename XP<N>::P;
+template <int N> using XPlan = dlfft::Narrow<N>;
 struct XArgs {
     double2 *P;          // [6][z][y][n/2]
     int nek;
@@ -94,6 +90,9 @@ template <int N>
 __host__ __device__ constexpr int x_units() { return N <= 64 ? (N == 32 ? 8 : 4) : 64 / XPlan<N>::T; }
 template <int N>
 __host__ __device__ constexpr int x_threads() { return 3 * XPlan<N>::T * x_units<N>(); }
+// blocks per SM that the registers are cut for: 80 a thread at 8 elements, 168 beyond
+template <int N>
+__host__ __device__ constexpr int x_blocks() { return dlfft::elems<XPlan<N>>() > 8 ? 2 : 4; }
 template <int N>
 __host__ __device__ constexpr int x_smem() { return x_units<N>() * 6 * slot_len<XPlan<N>>() * 16; }
 
@@ -116,7 +115,7 @@ __device__ __forceinline__ void emit_value(F *row, int x, int n, double u)
 // element and thread group (0.26 ms at 256^3), 1.6 GB of DRAM (0.25 ms); 0.47 ms, where the
 // library's x transforms and the cross-product kernel took 0.78.
 template <int N, int MODE>
-__global__ void __launch_bounds__(x_threads<N>(), N == 256 ? 2 : 4) k_xpass(XArgs A)
+__global__ void __launch_bounds__(x_threads<N>(), x_blocks<N>()) k_xpass(XArgs A)
 {
     using P = XPlan<N>;
     constexpr int H = N / 2, T = P::T, L = P::S - 1, E = dlfft::elems<P>();
