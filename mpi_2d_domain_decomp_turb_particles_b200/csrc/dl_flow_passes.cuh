@@ -175,16 +175,17 @@ __global__ void __launch_bounds__(x_threads<N>(), x_blocks<N>()) k_xpass(XArgs A
     if (MODE == X_DISS) {
         // lines 3..5 hold the off-diagonal strain e12, e23, e31, lines 0..2 the diagonal; the
         // reference's order (partlib.f90:4007-4080)
-        for (int j = p * T + t; j < 2 * N; j += 3 * T) {
-            const int r = j / N, x = j - r * N;
-            double s[6];
+        double *e = A.diss + ((int64_t)z * N + y0) * N;
+        for (int x = p * T + t; x < N; x += 3 * T) {
+            double2 s[6];
+            for (int c = 0; c < 6; c++) s[c] = reg[(c < 3 ? 3 + c : c - 3) * SL + at(x)];
+            double ea = 0.0, eb = 0.0;
             for (int c = 0; c < 6; c++) {
-                const double2 a = reg[(c < 3 ? 3 + c : c - 3) * SL + at(x)];
-                s[c] = r ? a.y : a.x;
+                ea = c < 3 ? ea + 2.0 * s[c].x * s[c].x : ea + s[c].x * s[c].x;
+                eb = c < 3 ? eb + 2.0 * s[c].y * s[c].y : eb + s[c].y * s[c].y;
             }
-            double e = 0.0;
-            for (int c = 0; c < 6; c++) e = c < 3 ? e + 2.0 * s[c] * s[c] : e + s[c] * s[c];
-            A.diss[((int64_t)z * N + y0 + r) * N + x] = A.nu2 * e;
+            e[x] = A.nu2 * ea;
+            e[N + x] = A.nu2 * eb;
         }
         return;
     }
