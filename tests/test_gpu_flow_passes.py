@@ -168,3 +168,65 @@ def test_plane_flow_stays_plane(n, c):
     for zero, whole in parts:
         assert float(zero.norm() / whole.norm()) <= (TOL if c == 1 else 0.0)
     g.close()
+
+
+@pytest.mark.parametrize("n", [32, 96, 128, 192, 256, 384, 512])
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_emission_of_every_plan(n, precision):
+    """As above for every plan and barrier form of the x pass, with droplets at the faces."""
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    g = Flow(n, 1e-3, 1e-4)
+    g.set_velocity(torch.randn((3, n, n, n), generator=gen, device="cuda", dtype=torch.float64))
+    d = [Partlib(dense_params(n=n, npart=4000, precision=precision)) for _ in range(2)]
+    rng = np.random.default_rng(n)
+    faces = rng.choice([0.0, 1e-9, 2 * np.pi - 1e-9], (1000, 3))
+    for p in d:
+        p.part_init()
+        yp = p.get_particles()["yp"]
+        yp[:1000, :3] = faces
+        p.set_particles(yp)
+    g.step(d[0])
+    d[1].set_fields(*g.velocity_tensors())
+    for p in d:
+        p.update_step()
+    a, b = (p.get_particles() for p in d)
+    assert a["fdp"].any() and all(np.array_equal(a[k], b[k]) for k in a)
+    for p in d:
+        p.close()
+    g.close()
+
+
+@pytest.mark.parametrize("n", [384, 512])
+def test_dissipation_and_forced_step_of_the_largest_grids(n):
+    """DISSIP and the update with the deterministic forcing against torch."""
+    nu, dt, force = 1e-2, 1e-3, (0.3, 0.2)
+    gen = torch.Generator(device="cuda").manual_seed(6)
+    kv, _ = wavenumbers(n)
+    g = Flow(n, nu, dt, forcing=1, force=force)
+    g.set_velocity(torch.randn((3, n, n, n), generator=gen, device="cuda", dtype=torch.float64))
+    uh = torch.from_numpy(g.spectral()[0]).cuda()
+    diss = torch.zeros((n, n, n), dtype=torch.float64, device="cuda")
+    for a in range(3):
+        for b in range(a + 1):
+            s = torch.fft.irfftn(0.5j * (kv[a] * uh[b] + kv[b] * uh[a]), s=(n,) * 3, norm="forward")
+            diss += 2 * nu * (1 if a == b else 2) * s * s
+    t = g.dissipation_tensor()
+    assert float((t - diss).norm() / diss.norm()) < TOL
+    del diss, s
+    g.step()
+    new, nold = (torch.from_numpy(v).cuda() for v in g.spectral())
+    k2 = kv[0] ** 2 + kv[1] ** 2 + kv[2] ** 2
+    shell = (k2 > 0).int() * ((k2 <= 2).int() + ((k2 > 2) & (k2 <= 6)).int() * 2)
+    k2[0, 0, 0] = 1e-5
+    # N_old of the first step is the state itself
+    v = uh * (1 - 0.5 * nu * dt * k2) + dt * (1.5 * nold - 0.5 * uh)
+    div = (kv[0] * v[0] + kv[1] * v[1] + kv[2] * v[2]) / k2
+    v = torch.stack([v[c] - kv[c] * div for c in range(3)]) / (1 + 0.5 * nu * dt * k2)
+    e = (v.abs() ** 2).sum(0)
+    e[:, :, 0] *= 0.5
+    for q in (1, 2):
+        v = torch.where(shell == q, v * (force[q - 1] / e[shell == q].sum()).sqrt(), v)
+    v[:, 0, 0, 0] = 0.0
+    assert float((new - v).norm() / v.norm()) < TOL
+    assert float((torch.where(shell > 0, new - v, 0.0)).norm() / torch.where(shell > 0, v, 0.0).norm()) < TOL
+    g.close()
