@@ -1389,22 +1389,25 @@ extern "C" int dl_adj_set_droplets(dl_adj *a, const double *x0, const double *ta
 {
     if (!a || !x0 || !tau || !radius) return DL_E_ARG;
     const int np = a->p.np;
-    const double *dx = x0, *dtau = tau, *drad = radius;
-    double *tmp = nullptr;
+    const size_t b = sizeof(double) * (size_t)np;
+    // The inputs are copied, not read in place: the copy checks their ranges.  They go to the
+    // recorded trajectory's buffer (15 np doubles at least), which is free between calls.
+    double *dx = a->TX, *dtau = dx + 3 * (size_t)np, *drad = dtau + np;
     if (on_device) {
+        for (const double *q : {x0, tau, radius}) {
+            cudaPointerAttributes at;
+            ACUDA(a, cudaPointerGetAttributes(&at, q));
+            if (at.type == cudaMemoryTypeUnregistered)
+                return afail(a, DL_E_ARG, "dl_adj_set_droplets: on_device with a host pointer");
+        }
         // inputs written on the legacy stream (or a blocking one) come first
         ACUDA(a, cudaEventRecord(a->ev[0], cudaStreamLegacy));
         ACUDA(a, cudaStreamWaitEvent(a->stream, a->ev[0], 0));
-    } else {
-        ACUDA(a, cudaMallocAsync((void **)&tmp, sizeof(double) * 5 * (size_t)np, a->stream));
-        const size_t b = sizeof(double) * (size_t)np;
-        ACUDA(a, cudaMemcpyAsync(tmp, x0, 3 * b, cudaMemcpyHostToDevice, a->stream));
-        ACUDA(a, cudaMemcpyAsync(tmp + 3 * (size_t)np, tau, b, cudaMemcpyHostToDevice, a->stream));
-        ACUDA(a, cudaMemcpyAsync(tmp + 4 * (size_t)np, radius, b, cudaMemcpyHostToDevice, a->stream));
-        dx = tmp;
-        dtau = tmp + 3 * (size_t)np;
-        drad = tmp + 4 * (size_t)np;
     }
+    const cudaMemcpyKind kind = on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
+    ACUDA(a, cudaMemcpyAsync(dx, x0, 3 * b, kind, a->stream));
+    ACUDA(a, cudaMemcpyAsync(dtau, tau, b, kind, a->stream));
+    ACUDA(a, cudaMemcpyAsync(drad, radius, b, kind, a->stream));
     // internal order: droplets sorted along the Morton curve of the cells of their initial
     // position, so that the stencils of a warp cover a compact box (shared cache lines in
     // the gathers, nearby grid points in the gradient atomics)
@@ -1426,7 +1429,6 @@ extern "C" int dl_adj_set_droplets(dl_adj *a, const double *x0, const double *ta
     ACUDA(a, cudaMemsetAsync(a->rmax, 0, sizeof(double), a->stream));
     k_rad_max<<<std::min(296, dl_blocks(np, 256)), 256, 0, a->stream>>>(np, a->rad, (unsigned long long *)a->rmax);
     ACUDA(a, cudaGetLastError());
-    if (tmp) ACUDA(a, cudaFreeAsync(tmp, a->stream));
     double rmax = 0.0;
     ACUDA(a, cudaMemcpyAsync(&rmax, a->rmax, sizeof(double), cudaMemcpyDeviceToHost, a->stream));
     ACUDA(a, cudaStreamSynchronize(a->stream));

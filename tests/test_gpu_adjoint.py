@@ -12,6 +12,7 @@ import pytest
 
 import oracle as orc
 from test_oracle_adjoint import clustered_case
+from mpi_2d_domain_decomp_turb_particles_b200._lib import DropletError
 from mpi_2d_domain_decomp_turb_particles_b200.adjoint import AdjointParams, DropletAdjoint, droplet_loss
 
 pytestmark = pytest.mark.gpu
@@ -207,4 +208,19 @@ def test_recomputation_repeats_the_forward_pass(np_):
     dtau = a.backward()[1]
     assert (s2 > 0.0).all()
     assert np.allclose(dtau, -2.0 * s2 / (np_ * tau * (1.0 + 9.0 * dt / (24.0 * tau))), rtol=1e-5, atol=0.0)
+    a.close()
+
+
+def test_droplets_partly_on_the_host_are_refused():
+    """Device positions with host drag times: an error, and the droplets set before stay."""
+    import torch
+    u, x0, tau, rad = clustered_case()
+    a = gpu_problem("fp64", u=u, x0=x0, tau=tau, rad=rad)
+    loss, _ = a.forward()
+    for q in (1, 2):
+        args = [torch.from_numpy(x0 + 0.5).cuda(), torch.from_numpy(tau).cuda(), torch.from_numpy(rad).cuda()]
+        args[q] = (x0, tau, rad)[q]
+        with pytest.raises(DropletError):
+            a.set_droplets(*args)
+    assert a.forward()[0] == loss
     a.close()
