@@ -27,14 +27,15 @@ template <> struct WideT<192> { using P = PlanOf<192, 16, 12, 16>; };
 template <> struct WideT<256> { using P = PlanOf<256, 16, 16, 16>; };
 template <> struct WideT<384> { using P = PlanOf<384, 64, 8, 8, 6>; };
 template <> struct WideT<512> { using P = PlanOf<512, 64, 8, 8, 8>; };
-// Narrow, for the x pass, is Wide but at 128 and 192, where it takes three stages of 8 elements
-// and twice the threads per line: the x pass holds six lines per pair of rows in shared memory,
-// which limits the threads per SM by lines rather than registers.  Flow step with the droplet
-// field, this and Wide: 128^3 203 and 225 us, 192^3 602 and 615.  At 96 the same form takes 101.5
-// and Wide 99.4; at 256 the steps are equal, and DISSIP takes 976 and 946.
+// Narrow, for the x pass: from 128 on three stages of 8 elements, with twice Wide's threads per
+// line up to 256: the x pass holds six lines per pair of rows in shared memory, which limits the
+// threads per SM by lines rather than registers.  Flow step with the droplet field, this and
+// Wide: 128^3 203 and 225 us, 192^3 602 and 615, 256^3 1,377 and 1,383.  At 96 the same form takes
+// 101.7 us and Wide 99.2.
 template <int N> struct NarrowT : WideT<N> {};
 template <> struct NarrowT<128> { using P = PlanOf<128, 16, 8, 4, 4>; };
 template <> struct NarrowT<192> { using P = PlanOf<192, 32, 8, 8, 3>; };
+template <> struct NarrowT<256> { using P = PlanOf<256, 32, 8, 8, 4>; };
 template <int N> using Wide = typename WideT<N>::P;
 template <int N> using Narrow = typename NarrowT<N>::P;
 

@@ -90,7 +90,7 @@ template <int N>
 __host__ __device__ constexpr int x_units() { return N <= 64 ? (N == 32 ? 8 : 4) : 64 / XPlan<N>::T; }
 template <int N>
 __host__ __device__ constexpr int x_threads() { return 3 * XPlan<N>::T * x_units<N>(); }
-// blocks per SM that the registers are cut for: 80 a thread at 8 elements, 168 beyond
+// blocks per SM that the registers are cut for: 80 a thread at 8 elements (168 at the 12 of 96)
 template <int N>
 __host__ __device__ constexpr int x_blocks() { return dlfft::elems<XPlan<N>>() > 8 ? 2 : 4; }
 template <int N>
@@ -111,9 +111,9 @@ __device__ __forceinline__ void emit_value(F *row, int x, int n, double u)
 // transforms along z and y have rounded its rows alike): beside another component a small one
 // would lose their ratio, and one that is zero would not stay so (and the components (0, 1) of a
 // row took 0.49 ms at 256^3).
-// Bound by the load/store unit and the latency of its phases: 24 16-byte accesses of the SM per
-// element and thread group (0.26 ms at 256^3), 1.6 GB of DRAM (0.25 ms); 0.47 ms, where the
-// library's x transforms and the cross-product kernel took 0.78.
+// Bound by the load/store unit and the latency of its phases: 31 16-byte accesses of the SM per
+// element and thread group with three stages (0.34 ms at 256^3), 1.6 GB of DRAM (0.25 ms); 0.47 ms,
+// where the library's x transforms and the cross-product kernel took 0.78.
 template <int N, int MODE>
 __global__ void __launch_bounds__(x_threads<N>(), x_blocks<N>()) k_xpass(XArgs A)
 {
