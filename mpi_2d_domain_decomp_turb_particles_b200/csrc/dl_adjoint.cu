@@ -1121,10 +1121,12 @@ int find_pairs(dl_adj *a)
         cudaFree(a->pairs);
         cudaFree(a->pair_refs);
         a->pairs = a->pair_refs = nullptr;
-        a->pair_cap = np2 + np2 / 4 + 1024;
-        int ra = aalloc(a, (void **)&a->pairs, sizeof(int2) * a->pair_cap);
-        if (!ra) ra = aalloc(a, (void **)&a->pair_refs, sizeof(int2) * a->pair_cap);
+        a->pair_cap = 0;   // until both are there: a failed call leaves nothing to write to
+        const int cap = np2 + np2 / 4 + 1024;
+        int ra = aalloc(a, (void **)&a->pairs, sizeof(int2) * cap);
+        if (!ra) ra = aalloc(a, (void **)&a->pair_refs, sizeof(int2) * cap);
         if (ra) return ra;
+        a->pair_cap = cap;
         return find_pairs<T>(a);
     }
     a->npairs = np2;
@@ -1153,6 +1155,7 @@ template <typename T>
 int forward_t(dl_adj *a, double *loss, int *npairs)
 {
     const int np = a->p.np;
+    a->forward_done = 0;   // the state and pairs of the last pass are rewritten
     ACUDA(a, cudaEventRecord(a->ev[0], a->stream));
     for (int seg = 0; seg < a->nseg; seg++) {
         int r = run_segment<T>(a, seg, false);
