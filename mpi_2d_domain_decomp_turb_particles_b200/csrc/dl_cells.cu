@@ -641,13 +641,9 @@ __device__ __forceinline__ void coll_pair(const CollArgs<T> &A, int4 r)
 }
 
 // Search pass: P threads per sorted entry (owners in cell order share their neighbour rows
-// in L1); the list goes through a block buffer, one global atomic per block.  One thread reads
-// its nine rows of cells one after the other, three dependent loads each; where the
-// droplets do not fill the chip several times over, four threads share the rows
-// (kCollSplit entries).
-// 20,000 droplets in 64^3 24 -> 12 us, 100,000 in 128^3 43 -> 30; at 200,000 both take 62, at
-// 1M one thread takes 200 and four 263
-constexpr int kCollSplit = 150000;
+// in L1; P = 4 by dl_split_rows); the list goes through a block buffer, one global atomic per
+// block.  One thread reads its nine rows of cells one after the other, three dependent loads
+// each.  At 1M in 256^3 one thread takes 200 us and four 263
 template <typename T, int P>
 __global__ void __launch_bounds__(128) k_coll_search(CollArgs<T> A)
 {
@@ -1268,7 +1264,7 @@ static int collision_t(dl_ctx *c, dl_coll_report *rep)
             nbz, ncount, c->nps, c->cand, c->coll_n, c->counts, c->hist_i, c->hist_d, c->coll_flag);
         DL_CHECK_LAUNCH(c);
         if (c->nps > 0) {
-            if (A.ne <= kCollSplit) k_coll_search<T, 4><<<dl_blocks(4 * (long)A.ne, t), t, 0, c->stream>>>(A);
+            if (dl_split_rows(A.ne, c->dc.ncd)) k_coll_search<T, 4><<<dl_blocks(4 * (long)A.ne, t), t, 0, c->stream>>>(A);
             else k_coll_search<T, 1><<<dl_blocks(A.ne, t), t, 0, c->stream>>>(A);
             DL_CHECK_LAUNCH(c);
             k_coll_eval<T><<<4 * c->num_sms, 256, 0, c->stream>>>(A);

@@ -157,11 +157,9 @@ __global__ void k_nei_scatter(int nnz, const NeiApp *app, const int *start, int 
 // truncation spheres leaves before the square root: the walk spends its time on instructions
 // of candidates that become no entry (256^3 / 1M with radii of 10 to 40 um: 312 -> 193 us in
 // perf/cases.py's coupled case, 204 -> 195 in the bench's; 512^3 / 5M lognormal to 60 um: 1.5 ms
-// as before).  9 CTAs per SM: 193 us, against 206 at 10 (spills), 197 at 8 and 209 at 7.
-// P threads share an owner's rows, as in the collision search: over few droplets one thread's
-// chain of rows is what the walk waits for (20,000 droplets in 64^3: 53 -> 21 us with four; both
-// take 19 at 100,000 in 128^3)
-constexpr int kWalkSplit = 150000;
+// as before).  9 CTAs per SM (56 registers, 52-56 bytes spilled): 193 us, against 206 at 10, 197
+// at 8 and 209 at 7.  P threads share an owner's rows, as in the collision search (P = 4 by
+// dl_split_rows; at 1M in 256^3 one thread takes 195 us and four 239)
 template <int P>
 __global__ void __launch_bounds__(128, 9) k_nei_walk(NeiArgs A)
 {
@@ -1904,7 +1902,7 @@ int launch_nei_list(dl_ctx *c)
         k_rad_max<<<std::min(dl_blocks(nps, 256), 4 * c->num_sms), 256, 0, c->stream>>>(nps, c->rad, d_napp + 1);
         DL_CHECK_LAUNCH(c);
         if (attempt) DL_CUDA(c, cudaMemsetAsync(c->nei_cnt, 0, sizeof(int) * (m + 1), c->stream));
-        if (A.ne <= kWalkSplit) k_nei_walk<4><<<dl_blocks(4 * (long)A.ne, 128), 128, 0, c->stream>>>(A);
+        if (dl_split_rows(A.ne, c->dc.ncd)) k_nei_walk<4><<<dl_blocks(4 * (long)A.ne, 128), 128, 0, c->stream>>>(A);
         else k_nei_walk<1><<<dl_blocks(A.ne, 128), 128, 0, c->stream>>>(A);
         DL_CHECK_LAUNCH(c);
         // CSR offsets and the largest count (the counts are complete even when the entry

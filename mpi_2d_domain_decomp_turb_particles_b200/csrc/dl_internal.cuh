@@ -371,3 +371,17 @@ double dl_ranff2(int *idum, int *iv, int *iy, int *idum2);
 
 // shared small utilities
 static inline int dl_blocks(long n, int t) { return (int)((n + t - 1) / t); }
+// Four threads per entry, sharing its rows of cells, instead of one in the searches over ne
+// cell-list entries.  One thread's chain of dependent loads is what a search waits for until the
+// entries fill the chip several times over, and the chain is the longer the more entries a
+// cell holds.  us of the collision search / neighbour walk, one thread and four:
+//   64^3    20,000  24 -> 12 / 53 -> 20     130,000  67 -> 70 / 155 -> 131
+//   96^3   100,000  50 -> 36 / 146 -> 115   130,000  55 -> 50 / 175 -> 146
+//   128^3  100,000  43 -> 30 / 20 -> 19     140,000  41 -> 42 / 20 -> 25
+//   256^3   75,000  19 -> 17 / 24 -> 22     100,000  21 -> 23 / 30 -> 31    140,000  23 -> 31 / 32 -> 37
+//   512^3   50,000  21 -> 17 / 56 -> 46     100,000  22 -> 22 / 53 -> 52
+static inline bool dl_split_rows(int ne, int ncd)
+{
+    const double per_cell = (double)ne / ((double)ncd * ncd * ncd);
+    return ne <= 150000 && ne <= 80000.0 + 800000.0 * per_cell;
+}

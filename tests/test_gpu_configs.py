@@ -17,6 +17,7 @@ import numpy as np
 import pytest
 
 import oracle as orc
+from cases import smooth_field
 from mpi_2d_domain_decomp_turb_particles_b200 import Partlib, ParticleParams
 from test_gpu_hdi import oracle_nei, through_nei
 from test_gpu_parity import _compare_collision, gpu_state, oracle_state
@@ -227,4 +228,26 @@ def test_config2_mixed_interpolation_and_hdi_step(c2_inputs):
     s = g.get_particles()
     ref = o.yp[:o.nps]
     assert np.linalg.norm(s["yp"][:, 3:6] - ref[:, 3:6]) <= 1e-5 * np.linalg.norm(ref[:, 3:6])
+    g.close()
+
+
+@pytest.mark.parametrize("n", [96, 192])
+def test_searches_on_either_side_of_their_split(n):
+    """95,000 droplets: four threads per droplet in the collision search and the neighbour
+    walk at 96^3, one at 192^3, where the cells hold fewer."""
+    f = smooth_field(n)
+    p = ParticleParams(precision="fp64", **dict(C2, nx=n, npart=95_000, etk_dns=0.02, tauk_dns=0.2))
+    g, o = _make(p, {"nei_max": C2["nei_max"]})
+    g.set_fields(*f)
+    for x in (g, o):
+        x.periodic()
+        x.overlap_det()
+    gm, rep, (nei, onei), pert, pairs, nir = _hdi_step_separate(g, o, f)
+    assert onei[1].shape[0] > 1000 and nir[1].sum() > 100
+    assert all(np.array_equal(a, b) for a, b in zip(nei, onei))
+    assert gm.iterations == o.geti("gmres_iter")
+    assert np.linalg.norm(pert[0] - pert[1]) <= 1e-10 * np.linalg.norm(pert[1])
+    assert rep.candidate_pairs == o.getl("candidate_pairs")
+    assert pairs[0] == pairs[1] and np.array_equal(*nir)
+    assert np.array_equal(g.removal_list(), o.removepart())
     g.close()
