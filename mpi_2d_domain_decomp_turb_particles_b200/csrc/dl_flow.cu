@@ -690,7 +690,8 @@ int finish(dl_flow *f)
     return f->fast ? transform_state(f, false) : 0;
 }
 
-// spectral state between the caller's layout (rows [z][y] of nh modes) and the context's
+// spectral state between the caller's layout (rows [z][y] of nh modes) and the context's; one
+// component per blockIdx.y
 __global__ void k_layout(Grid G, double2 *state, double2 *packed, int in)
 {
     const int64_t m = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -699,27 +700,24 @@ __global__ void k_layout(Grid G, double2 *state, double2 *packed, int in)
     double kx, ky, kz;
     mode_of(G, m, x, y, z, kx, ky, kz);
     if (x >= G.nh) return;
-    const int64_t q = ((int64_t)z * G.n + y) * G.nh + x;
-    if (in) state[m] = packed[q];
-    else packed[q] = state[m];
+    const int64_t rows = (int64_t)G.n * G.n, c = blockIdx.y;
+    double2 *s = state + c * G.M + m, *p = packed + (c * rows + (int64_t)z * G.n + y) * G.nh + x;
+    if (in) *s = *p;
+    else *p = *s;
 }
 
-// all three components, caller <-> state, through P where the layouts differ
+// all three components, caller <-> state, through P where the layouts differ (it is free between
+// steps and holds three packed components)
 int copy_state(dl_flow *f, double2 *state, void *caller, bool in, cudaMemcpyKind k)
 {
-    const int64_t packed = (int64_t)f->G.n * f->G.n * f->G.nh;
-    if (!f->fast) {
-        const size_t b = sizeof(double2) * 3 * packed;
-        FCUDA(f, in ? cudaMemcpyAsync(state, caller, b, k, f->stream) : cudaMemcpyAsync(caller, state, b, k, f->stream));
-        return 0;
-    }
-    for (int c = 0; c < 3; c++) {   // P is free between steps and holds three packed components
-        double2 *mine = static_cast<double2 *>(caller) + c * packed, *tmp = f->planes + c * packed;
-        if (in) FCUDA(f, cudaMemcpyAsync(tmp, mine, sizeof(double2) * packed, k, f->stream));
-        k_layout<<<blocks(f->G.M, 256), 256, 0, f->stream>>>(f->G, state + c * f->G.M, tmp, in);
+    const size_t b = sizeof(double2) * 3 * f->G.n * f->G.n * f->G.nh;
+    double2 *buf = f->fast ? f->planes : state;
+    if (in) FCUDA(f, cudaMemcpyAsync(buf, caller, b, k, f->stream));
+    if (f->fast) {
+        k_layout<<<dim3(blocks(f->G.M, 256), 3), 256, 0, f->stream>>>(f->G, state, buf, in);
         FCUDA(f, cudaGetLastError());
-        if (!in) FCUDA(f, cudaMemcpyAsync(mine, tmp, sizeof(double2) * packed, k, f->stream));
     }
+    if (!in) FCUDA(f, cudaMemcpyAsync(caller, buf, b, k, f->stream));
     return 0;
 }
 
