@@ -10,7 +10,8 @@ pass over the three field components: 3 n^3 * 4 B (mixed, FP32 field) or 3 n^3 *
 Of these the interpolation kernel moves the field, the positions it reads (24 B) and the
 velocity it writes (3 words); the advance kernel the rest.
 
-Flow step (FP64, M = n * n * (n/2 + 1) complex modes): the update kernel reads the
+Flow step on the grids that cuFFT transforms (FP64, M = n * n * (n/2 + 1) complex modes; the
+others: flow_pass_bytes): the update kernel reads the
 transformed product, N_old and u (3 components each) and writes N_old, u and the six
 inputs of the next transforms: 21 complex words = 336 B per mode.  The cross-product
 kernel reads u and omega (6 words) and writes u x omega (3 words) per point, 72 B, plus

@@ -19,8 +19,8 @@
 //     inputs [curl u^, u^] of the next step                          (flowlib.f90:180-334)
 // Grids 2^a and 3 * 2^a from 32 to 512 take the passes of dl_flow_passes.cuh, which transform
 // along one direction each, only inside the dealiasing sphere, with the cross product between
-// the two x transforms in shared memory: 256^3 2.12 -> 1.37 ms, 512^3 18.5 -> 11.4 ms,
-// 64^3 86 -> 48 us, 192^3 1.02 -> 0.59 ms.  Other grids take cuFFT's 3D transforms (Z2D / D2Z, batched
+// the two x transforms in shared memory: 256^3 2.12 -> 1.34 ms, 512^3 18.5 -> 11.4 ms,
+// 64^3 86 -> 46 us, 192^3 1.02 -> 0.59 ms, 32^3 67 -> 33 us.  Other grids take cuFFT's 3D transforms (Z2D / D2Z, batched
 // over components) with kernels for the cross product, the update and the finish.
 // Decision on a reference quirk: with one rank, symmetrize's test idlocalZ .eq. nprocZ/2
 // (flowlib.f90:253) is true for the rank holding ky = 0 and would zero the ky = 0 plane;

@@ -1196,7 +1196,6 @@ __global__ void __launch_bounds__(256) k_convert_field(const double *__restrict_
     }
 }
 
-// MEAN_VEL partial sums (partlib.f90:1910-1930) -> 11*nset doubles via FP64 atomics.
 // MEAN_VEL's eleven sums per radius set (partlib.f90:1889-1980): sum, sum of squares and
 // sum of magnitudes of each component, then of |(u_y, u_z)| and |u|.  Each thread adds its
 // droplets (a grid-stride range) into registers for kMvSets sets at a time, the block adds

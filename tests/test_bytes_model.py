@@ -33,3 +33,18 @@ def test_interp_onchip_floor():
     assert abs(f["floor_ms"] - f["fp64_ops"] / (148 * 64 * 1965e6) * 1e3) < 1e-12
     # without a clock record the nominal maximum clock is used
     assert bm.interp_onchip("mixed", 10, 1.0, 148, None)["sm_mhz"] == 1965.0
+
+
+def test_flow_pass_bytes():
+    """The dealiased share counted mode by mode: the formula's circle and sphere are its areas."""
+    import numpy as np
+    for n in (64, 128, 256):
+        nek = int(n / 2 - 1.5)
+        k = np.fft.fftfreq(n, 1.0 / n)
+        h2 = np.arange(n // 2) ** 2 + (k ** 2)[:, None]
+        circle = np.count_nonzero(h2 <= nek * (nek + 1))
+        sphere = sum(np.count_nonzero(h2 + q * q <= nek * (nek + 1)) for q in k)
+        x = 9 * 16 * n * n * (n // 2) + (24 + 12) * n ** 3
+        update = 16 * (18 * sphere + 6 * n * circle)
+        got = bm.flow_pass_bytes(n)
+        assert got["x"] == x and abs(got["update"] - update) < 0.03 * update
