@@ -346,7 +346,9 @@ int dl_flow_dissipation(dl_flow *f, const double **field);
  * Loss = w_wr * mean over final pairs |r| < pair_factor * (a_i + a_j) (minimum image) of
  * (v_i - v_j) . r / |r|  +  w_disp * mean over droplets of |x(T) - x(0)|^2.
  * The forward pass keeps a checkpoint every checkpoint_every steps; the backward pass
- * recomputes each segment from its checkpoint and runs the exact discrete adjoint. */
+ * recomputes each segment from its checkpoint, bit for bit, and runs the exact discrete
+ * adjoint.  DL_MIXED rounds the velocities to FP32 at the checkpoints (between them they are
+ * updated in FP64), so there the interval shows in the last FP32 bits of the results. */
 typedef struct dl_adj_params {
     int n;                       /* grid points per side */
     int np;                      /* droplets */

@@ -224,3 +224,27 @@ def test_droplets_partly_on_the_host_are_refused():
             a.set_droplets(*args)
     assert a.forward()[0] == loss
     a.close()
+
+
+@pytest.mark.parametrize("seed", [0, 1])
+def test_mixed_velocity_takes_no_rounding_per_step(seed):
+    """Mixed: the droplet velocity after 100 steps of slow drag is as far from FP64 as one
+    interpolation and one stored FP32 value round, about 1e-7, and not as 100 updates in FP32
+    do (1e-6 and more here); 3e-7 lies between."""
+    rng = np.random.default_rng(seed)
+    n, np_ = 16, 300
+    x = np.arange(n) * (2 * np.pi / n)
+    Z, Y, X = np.meshgrid(x, x, x, indexing="ij")
+    u = np.stack([sum(rng.standard_normal() * np.cos(k[0] * X + k[1] * Y + k[2] * Z + rng.uniform(0, 6.28))
+                      for k in rng.integers(-3, 4, (8, 3))) for _ in range(3)])
+    x0, tau = rng.uniform(0, 2 * np.pi, (np_, 3)), rng.uniform(1.0, 3.0, np_)
+    v = {}
+    for prec in ("fp64", "mixed"):
+        a = DropletAdjoint(AdjointParams(n=n, nsteps=100, dt=0.01, gravity=1.0, precision=prec,
+                                         checkpoint_every=100, pair_factor=0.0), np_)
+        a.set_field(u)
+        a.set_droplets(x0, tau, np.full(np_, 1e-6))
+        a.forward()
+        v[prec] = a.final_state()[1]
+        a.close()
+    assert np.linalg.norm(v["mixed"] - v["fp64"]) < 3e-7 * np.linalg.norm(v["fp64"])
