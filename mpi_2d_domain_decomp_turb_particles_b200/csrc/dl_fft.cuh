@@ -246,7 +246,7 @@ __device__ __forceinline__ void each(int t, F f)
 
 // tw: for each stage after the first, w^(m q) at (m - 1) * NS + q (contiguous in q, the
 // index neighbouring threads differ in).  Reading a quarter of the powers and multiplying the
-// rest from them was no faster in any pass (x at 256^3: 0.58 against 0.49 ms).
+// rest from them was no faster in any pass (x at 256^3, in two stages: 0.58 against 0.49 ms).
 template <class P, int SIGN, int s>
 __device__ __forceinline__ void butterflies(int t, double2 *v, const double2 *__restrict__ tw)
 {
